@@ -344,8 +344,12 @@ int sfwi_set_source(sfwi_handle *h, int kind);
 #define SFWI_TILE_8x32_2CELL_3STAGE 5
 #define SFWI_NUM_TILE_SHAPES 6
 
-/* Select the tile shape for this handle's runs.  Until one is selected (here
- * or by sfwi_autotune) each batch gets SFWI_TILE_16x32, or
+/* Select the tile shape for this handle's runs, which then take the four
+ * sweeps of a time step as launches of their own.  Until one is selected here,
+ * batches that gain from it run whole time steps per launch (sfwi_march.cu, chosen by
+ * the batch's size; it takes a second copy of the wavefields where memory
+ * is plentiful), with the same results bit for bit; other batches run the
+ * sweeps.  Until a shape is selected (here or by sfwi_autotune) each batch gets SFWI_TILE_16x32, or
  * SFWI_TILE_8x32_2CELL_3STAGE when its 16x32 tiles would give fewer than four
  * to each of the device's CTA slots (small batches).  A batch already on
  * the device is re-tiled.  Results do not depend on the shape: they are
@@ -370,7 +374,8 @@ int sfwi_get_tile_shape(sfwi_handle *h, int *shape, int *tx, int *tz);
  * step of the four step kernels for every tile shape on the resident batch
  * (reps steps each, as sfwi_time_kernels) and keep the fastest.  *choice gets
  * its SFWI_TILE_* index, out_ms (optional, SFWI_NUM_TILE_SHAPES floats) the
- * per-step time of each shape.  Like sfwi_time_kernels it overwrites the
+ * per-step time of each shape; batches that run whole time steps per launch
+ * keep doing so.  Like sfwi_time_kernels it overwrites the
  * last run's wavefields; its gradients, already accumulated, are untouched. */
 int sfwi_autotune(sfwi_handle *h, int reps, int *choice, float *out_ms);
 /* page-locked host buffers (cudaMallocHost) for records that are copied every

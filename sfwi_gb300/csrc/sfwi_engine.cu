@@ -13,6 +13,7 @@
 #include <string>
 #include <vector>
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <mutex>
 
@@ -232,6 +233,18 @@ struct Batch {
     DevBuf<int> derr;        // device-side error flag (bounded waits)
     DevBuf<int> dctr;        // dynamic tile counters of the step kernels (zeroed per run)
     TmaMaps tm;              // tensor maps of `grid` for the current X, P
+    // whole time steps per launch (sfwi_march.cu), forward and backward: the way
+    // they take (null: the sweeps), the second copy of the fields, the items,
+    // tensor maps reading either copy
+    const MarchVariant *way[2] = {nullptr, nullptr};
+    DevBuf<float> grid2;     // further copies of the fields, and the PML factors
+    float *fwd_copy[2] = {nullptr, nullptr}, *bwd_copy[2] = {nullptr, nullptr};
+    bool fwd_pairs = false, bwd_pairs = false;  // two fields as float2 per cell
+    float *fx = nullptr, *fz = nullptr;  // PML factors
+    std::vector<MarchItem> items[2];   // forward, backward
+    std::vector<int> items_active[2];  // per time step: items of the shots still running (empty: all)
+    DevBuf<MarchItem> ditems;          // both tables, back to back
+    MarchMaps mf[2], mb[2];  // forward and backward steps reading copy 0 or 1
     // graphs of the time loops for the current shape
     cudaGraphExec_t gfwd = nullptr, gbwd = nullptr;
     std::vector<long long> gsig;  // shape signature of the captured graphs
@@ -280,6 +293,7 @@ struct sfwi_handle {
     bool last_forward_only = false;
     const TileVariant *tv = nullptr;  // tile shape of the step kernels
     bool tile_auto = true;            // shape picked per batch by its size (until one is set)
+    bool march_ok = true;             // large enough batches may run whole steps per launch
     int nsm = 0;                      // multiprocessors of the device
     // trial models of a line search: while set, shots cut their windows from
     // these slot arrays instead of the uploaded model
@@ -352,17 +366,19 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     return fn;
 }
 
-// 3-D tiled map over the packed grid: dims (P, X, NGRID) floats, boxes of
+// 3-D tiled map over the packed grid: dims (P, X, narr) floats (pairs: float2s), boxes of
 // bz x bx x depth (depth consecutive arrays); out-of-range elements of a box
 // load arrive as zeros
-int encode_grid_map(CUtensorMap *m, float *base, int P, int X, int bz, int bx, int depth) {
+int encode_grid_map(CUtensorMap *m, float *base, int P, int X, int bz, int bx, int depth, int narr = NGRID,
+                    bool pairs = false) {
     auto enc = tensor_map_encoder();
     if (!enc) return fail(SFWI_E_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-    const cuuint64_t dims[3] = {(cuuint64_t)P, (cuuint64_t)X, (cuuint64_t)NGRID};
-    const cuuint64_t strides[2] = {(cuuint64_t)P * 4, (cuuint64_t)P * X * 4};
+    const cuuint64_t dims[3] = {(cuuint64_t)P, (cuuint64_t)X, (cuuint64_t)narr};
+    const cuuint64_t es = pairs ? 8 : 4;
+    const cuuint64_t strides[2] = {(cuuint64_t)P * es, (cuuint64_t)P * X * es};
     const cuuint32_t box[3] = {(cuuint32_t)bz, (cuuint32_t)bx, (cuuint32_t)depth};
     const cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box, estr,
+    CUresult r = enc(m, pairs ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(SFWI_E_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
@@ -630,6 +646,322 @@ int encode_tile_maps(sfwi_handle *h, bool forward_only) {
     return encode_2d_map(&b.tm.rs, b.rsrc.p, b.rsp, b.X, 4, bx);
 }
 
+// Whole time steps per launch (sfwi_march.cu).  Where the two copies of the
+// fields live.  Plain fields are ten arrays (the adjoint alone: eight), pairs
+// twenty; a copy takes the arrays of `grid` that the run does not use
+// otherwise, or arrays of `grid2`, which ends with the PML factors.
+size_t layout_march(sfwi_handle *h, bool forward_only) {
+    Batch &b = h->b;
+    const bool born = h->stage == 2, snap = !forward_only && h->snap_every > 0;
+    size_t n2 = 0;  // arrays of grid2
+    auto in_grid = [&](int k) { return b.grid.p + (size_t)k * b.cells; };
+    auto in_grid2 = [&](int n) {
+        float *q = b.grid2.p + n2 * b.cells;
+        n2 += n;
+        return q;
+    };
+    b.fwd_copy[0] = b.fwd_copy[1] = b.bwd_copy[0] = b.bwd_copy[1] = nullptr;
+    b.fwd_pairs = b.way[0] && born;
+    if (b.way[0]) {
+        // (backward sweeps start from plain fields in `grid`)
+        const bool to_sweeps = born && !forward_only && !snap && !b.way[1];
+        b.fwd_copy[0] = to_sweeps ? in_grid2(20) : in_grid(BG_VX);
+        b.fwd_copy[1] = born ? in_grid2(20) : in_grid(SC_VX);
+    }
+    b.bwd_pairs = b.way[1] && !snap;
+    if (b.bwd_pairs) {
+        b.bwd_copy[0] = b.fwd_pairs ? b.fwd_copy[0] : in_grid2(20);
+        b.bwd_copy[1] = b.fwd_pairs ? b.fwd_copy[1] : in_grid2(20);
+    } else if (b.way[1]) {
+        b.bwd_copy[0] = in_grid(AD_VX);
+        b.bwd_copy[1] = in_grid2(8);
+    }
+    b.fx = in_grid2(2);
+    b.fz = in_grid2(2);
+    return n2 * b.cells;
+}
+
+// The items of a step for strips of at most ps - 16 columns on `slots` CTA
+// slots: every shot's update region in strips of equal width (a multiple of
+// four columns, as the boxes start on 16 bytes) and runs of rows of equal cost, the
+// cost that a few full waves of items cover the batch with.  A run costs
+// its rows and about MARCH_FILL more (the rim above and below it, the ring's
+// first fill); rows in the x-PML cost MARCH_EDGE, strips that hold z-PML
+// columns MARCH_SIDE times as much.
+constexpr double MARCH_FILL = 14.0, MARCH_EDGE = 1.6, MARCH_SIDE = 1.25;
+struct Strip {
+    int z0, zw;
+    double side;
+};
+std::vector<Strip> march_strips(const ShotGeo &g, int pc, int pml) {
+    const int cols = g.nzpml - 2 * NOP, n = (cols + pc - 1) / pc, w = ((cols + n - 1) / n + 3) & ~3;
+    std::vector<Strip> v;
+    for (int z0 = NOP; z0 < g.nzpml - NOP; z0 += w) {
+        const int zw = std::min(w, (g.nzpml - NOP - z0 + 3) & ~3);
+        v.push_back(Strip{z0, zw, z0 < pml || z0 + zw > g.nzpml - pml ? MARCH_SIDE : 1.0});
+    }
+    return v;
+}
+// items of a burst with runs of `rows` rows
+long long burst_count(const sfwi_handle *h, const MarchVariant &w, int rows) {
+    long long n = 0;
+    for (const ShotGeo &g : h->b.geo)
+        n += (long long)march_strips(g, w.ps - 16, h->pml).size() * ((g.nxpml - 2 * NOP + rows - 1) / rows);
+    return n;
+}
+void march_items(const sfwi_handle *h, const MarchVariant &w, int slots, std::vector<MarchItem> &items,
+                 std::vector<int> &active) {
+    const Batch &b = h->b;
+    const int ps = w.ps, pc = ps - 16, pml = h->pml;
+    const bool burst = w.burst;
+    // cost of the rows [NOP, x) of a shot, in plain rows
+    auto rows_cost = [&](const ShotGeo &g, int x) {
+        const int e = pml + NOP, f = g.nxpml - pml - NOP;  // rows outside [e, f) are edge rows
+        const int n = std::max(0, std::min(x, g.nxpml - NOP) - NOP);
+        const int inner = std::max(0, std::min(x, f) - e);
+        return n + (MARCH_EDGE - 1.0) * (n - std::min(n, inner));
+    };
+    std::vector<std::vector<Strip>> st;
+    std::vector<double> tot;
+    for (const ShotGeo &g : b.geo) {
+        st.push_back(march_strips(g, pc, pml));
+        tot.push_back(rows_cost(g, g.nxpml));
+    }
+    double best = 8, cost = 0;
+    if (burst) {
+        // the shortest runs that still give every slot one item
+        for (best = G_ROWS; best < BURST_ROWS && burst_count(h, w, (int)best) > slots;) best += G_ROWS;
+    } else {
+        for (double len = 4; len <= 1024; len *= 1.02) {
+            long long n = 0;
+            double longest = 0;
+            for (int s = 0; s < b.nshots; s++)
+                for (const Strip &q : st[s]) {
+                    const double k = std::ceil(tot[s] * q.side / len);
+                    n += (long long)k;
+                    longest = std::max(longest, tot[s] * q.side / k);
+                }
+            const double c = (double)((n + slots - 1) / slots) * (longest + MARCH_FILL);
+            if (len == 4 || c < cost) cost = c, best = len;
+        }
+    }
+    items.clear();
+    active.clear();
+    std::vector<int> per_shot(b.nshots, 0);
+    for (int s = 0; s < b.nshots; s++) {
+        const ShotGeo &g = b.geo[s];
+        // the strips' runs side by side: neighbouring strips share rim columns
+        std::vector<std::vector<int>> cut(st[s].size());
+        size_t most = 0;
+        for (size_t q = 0; q < st[s].size(); q++) {
+            int x = NOP;
+            cut[q].push_back(x);
+            if (burst) {
+                while (x < g.nxpml - NOP) cut[q].push_back(x += (int)best);
+                cut[q].back() = g.nxpml - NOP;
+                most = std::max(most, cut[q].size());
+                continue;
+            }
+            const int k = (int)std::ceil(tot[s] * st[s][q].side / best);
+            for (int r = 1; r <= k; r++) {
+                // whole groups, so that only a strip's last run has a part of one
+                const double want = tot[s] * r / k;
+                int y = x;
+                while (y < g.nxpml - NOP && (r == k || rows_cost(g, y + 2) < want)) y += 4;
+                if (y > x) cut[q].push_back(x = y);
+            }
+            cut[q].back() = g.nxpml - NOP;
+            most = std::max(most, cut[q].size());
+        }
+        for (size_t r = 0; r + 1 < most; r++)
+            for (size_t q = 0; q < st[s].size(); q++) {
+                if (r + 1 >= cut[q].size()) continue;
+                MarchItem m{};
+                m.shot = s;
+                m.x0 = cut[q][r];
+                m.x1 = cut[q][r + 1];
+                m.z0 = st[s][q].z0;
+                m.zw = st[s][q].zw;
+                m.g = g;
+                const int v0 = m.x0 - 8, v1 = v0 + ((m.x1 - m.x0 + 3) / 4 + 4) * 4;
+                if (g.isx >= v0 && g.isx < v1 && g.isz >= m.z0 - 8 && g.isz < m.z0 - 8 + ps) m.flags |= MARCH_SOURCE;
+                if (g.ntr > 0 && g.igz >= m.z0 - 8 && g.igz < m.z0 - 8 + ps) m.flags |= MARCH_RECV;
+                items.push_back(m);
+                per_shot[s]++;
+            }
+    }
+    bool uneven = false;
+    for (const ShotAux &a : b.aux) uneven |= a.nt != h->nt;
+    if (uneven) {
+        // shots in order of decreasing nt: a step takes the items of those still running
+        active.assign(h->nt, 0);
+        for (int s = 0; s < b.nshots; s++)
+            for (int it = 0; it < b.aux[s].nt; it++) active[it] += per_shot[s];
+    }
+}
+
+void no_march(Batch &b) {
+    b.way[0] = b.way[1] = nullptr;
+    b.fwd_pairs = b.bwd_pairs = false;
+    for (int d = 0; d < 2; d++) b.items[d].clear(), b.items_active[d].clear();
+}
+// Decide whether the batch runs whole steps per launch, and plan it.  Per
+// step, sweeps -> whole step, 152 SMs (stage 1 / Born forward; backward):
+//   one wave of bursts, every SM at most one item (376x201, one shot): 8.3 -> 5.7 /
+//     9.8 -> 7.1; 11.1 -> 8.2 us.  Two waves (two shots) lose: 10.2 -> 10.4,
+//     13.5 -> 15.0 us.
+//   forward march, larger batches: 2 shots 10.2 -> 8.8 / 12.0 -> 11.2, 4 shots 15.3 -> 12.2 /
+//     18.8 -> 14.4, 12 shots 26.0 -> 23.9 / 36.0 -> 35.0, 38 shots 67 -> 62 / 107 -> 92 us.
+//     Below 2,000 cells an SM strips that are far from full lose (five shots of 153
+//     columns, two strips of 80: 9.4 -> 10.4; three of 183, two of 92: 9.0 -> 8.3).  Born
+//     between 8,000 and 15,000 cells an SM it depends on how the runs divide (ten
+//     shots at 401x301: 42.7 -> 44.2, uneven apertures 56.5 -> 55.7 us): sweeps
+//   backward march, pairs: the fill of the rings and the recomputed rim are a
+//     constant cost per item, so it pays from about 15,000 cells an SM (7,500:
+//     41.1 -> 43.6, 13,500: 65.2 -> 69.0, 15,000: 78.7 -> 75.2, 24,000: 121 -> 111 us)
+//   snapshots are launches of their own here and part of the sweeps there.  Nine
+//     shots at 376x201, every 1, 2, 4 steps: adjoint 23.9 -> 30.2, 22.5 -> 23.9,
+//     21.7 -> 20.5; Born forward 29.4 -> 33.0, 28.8 -> 30.2, 28.4 -> 28.8 (38 shots: as
+//     without); stage 1 forward in FP32 22.3 -> 21.4 but 13.1 -> 13.6 us with three
+//     shots, in 16 bits 25.2 -> 21.5, 23.2 -> 20.2, 22.4 -> 19.2 us
+// Grids of less than 64 cells an SM stay with the sweeps: such a step is all
+// launch latency, and the launch counts of the golden cases are the sweeps'.
+constexpr long long MARCH_MIN_CELLS = 64, MARCH_ANY_CELLS = 2000, MARCH_MID_CELLS = 8000, MARCH_LARGE_CELLS = 15000;
+constexpr int MARCH_SNAP_EVERY = 4;
+void plan_march(sfwi_handle *h, bool forward_only) {
+    Batch &b = h->b;
+    no_march(b);
+    // (a cell's offset is computed in 32 bits)
+    if (!h->march_ok || (long long)b.X * b.P >= (1LL << 31)) return;
+    const bool born = h->stage == 2, snap = h->snap_every > 0;
+    long long cells = 0, room = 0;  // room: cells of full strips
+    const int pc = march_wide()->ps - 16;
+    for (const ShotGeo &g : b.geo) {
+        const int rows = g.nxpml - 2 * NOP, cols = g.nzpml - 2 * NOP;
+        cells += (long long)rows * cols;
+        room += (long long)rows * ((cols + pc - 1) / pc * pc);
+    }
+    const long long per_sm = cells / std::max(h->nsm, 1);
+    if (per_sm < MARCH_MIN_CELLS) return;
+    const bool one_wave = burst_count(h, *march_burst(), BURST_ROWS) <= h->nsm, large = per_sm >= MARCH_LARGE_CELLS;
+    const bool taken = !forward_only && snap;  // snapshots are stored
+    const int every = taken ? h->snap_every : INT_MAX;
+    const bool fits = one_wave || per_sm >= MARCH_ANY_CELLS || 10 * cells >= 7 * room;
+    const bool fwd = !fits ? false
+                     : born ? (per_sm < MARCH_MID_CELLS || large) && every >= MARCH_SNAP_EVERY
+                            : every > 1 || h->snap_fmt != SNAP_F32;
+    const bool bwd = taken ? every >= MARCH_SNAP_EVERY : one_wave || large;
+    const MarchVariant *way = one_wave ? march_burst() : march_wide();
+    if (fwd) b.way[0] = way;
+    if (bwd && !forward_only) b.way[1] = way;
+    for (int d = 0; d < 2; d++)
+        if (const MarchVariant *w = b.way[d])
+            march_items(h, *w, h->nsm * (d ? w->bwd_ctas[!taken] : w->fwd_ctas[born]), b.items[d], b.items_active[d]);
+}
+
+// The second copy of the fields, the item tables and the tensor maps.  The
+// copy is taken only where memory is plentiful (an eighth of what is free): the run
+// takes the sweeps otherwise, which need none.
+int upload_march(sfwi_handle *h, bool forward_only) {
+    Batch &b = h->b;
+    if (!b.way[0] && !b.way[1]) return SFWI_OK;
+    const size_t n = layout_march(h, forward_only);
+    bool have = n <= b.grid2.n && b.grid2.p;
+    if (!have) {
+        size_t free_bytes = 0, total = 0;
+        b.grid2.release();
+        CK(cudaMemGetInfo(&free_bytes, &total));
+        have = n * sizeof(float) <= free_bytes / 8 && b.grid2.ensure(n) == cudaSuccess;
+    }
+    if (!have) {
+        no_march(b);
+        return SFWI_OK;
+    }
+    layout_march(h, forward_only);  // now with the buffer in place
+    CK(cudaMemsetAsync(b.grid2.p, 0, n * sizeof(float), h->st));
+    const size_t nf = b.items[0].size(), nb = b.items[1].size();
+    CK(b.ditems.ensure(nf + nb));
+    if (nf) CK(cudaMemcpyAsync(b.ditems.p, b.items[0].data(), nf * sizeof(MarchItem), cudaMemcpyHostToDevice, h->st));
+    if (nb) CK(cudaMemcpyAsync(b.ditems.p + nf, b.items[1].data(), nb * sizeof(MarchItem), cudaMemcpyHostToDevice, h->st));
+    for (int c = 0; c < 2; c++)
+        for (int back = 0; back < 2; back++) {
+            if (!b.way[back]) continue;
+            const int ps = b.way[back]->ps;
+            float *base = back ? b.bwd_copy[c] : b.fwd_copy[c];
+            const bool pairs = back ? b.bwd_pairs : b.fwd_pairs;
+            MarchMaps &m = back ? b.mb[c] : b.mf[c];
+            const int na = back && !pairs ? 8 : 10;
+            struct {
+                CUtensorMap *map;
+                int cols, depth;
+            } want[] = {{&m.view3, ps, 3}, {&m.view2, ps, 2}, {&m.rim3, ps - 8, 3}, {&m.rim2, ps - 8, 2}, {&m.core2, ps - 16, 2}};
+            for (auto &w : want)
+                if (int rc = encode_grid_map(w.map, base, b.P, b.X, w.cols, 4, w.depth, na, pairs)) return rc;
+            struct {
+                CUtensorMap *map;
+                int cols, depth;
+            } coef[] = {{&m.rim2c, ps - 8, 2}, {&m.rim1c, ps - 8, 1}, {&m.core2c, ps - 16, 2}, {&m.core1c, ps - 16, 1}};
+            for (auto &w : coef)
+                if (int rc = encode_grid_map(w.map, b.grid.p, b.P, b.X, w.cols, 4, w.depth)) return rc;
+        }
+    return SFWI_OK;
+}
+
+// the fields of one copy: ten arrays of `cells` cells of one or two floats
+FieldSet field_set(float *base, size_t cells, bool pairs) {
+    auto at = [&](int k) { return base + (size_t)k * cells * (pairs ? 2 : 1); };
+    return FieldSet{at(0), at(1), at(2), at(3), at(4), at(5), at(6), at(7), at(8), at(9)};
+}
+// the adjoint alone: no x-parts of txx and tzz
+FieldSet adjoint_set(float *base, size_t cells) {
+    auto at = [&](int k) { return base + (size_t)(k - AD_VX) * cells; };
+    return FieldSet{at(AD_VX), at(AD_VZ), at(AD_TXX), at(AD_TZZ), at(AD_TXZ),
+                    at(AD_MVX), at(AD_MVZ), nullptr, nullptr, at(AD_MTXZ)};
+}
+MarchArgs march_args(sfwi_handle *h, const Params &p, int rd, bool backward) {
+    Batch &b = h->b;
+    MarchArgs a{};
+    a.p = p;
+    if (!backward || b.bwd_pairs) {
+        float **copy = backward ? b.bwd_copy : b.fwd_copy;
+        const bool pairs = backward ? b.bwd_pairs : b.fwd_pairs;
+        a.p.bg = field_set(copy[rd ^ 1], b.cells, pairs);
+        a.in_bg = field_set(copy[rd], b.cells, pairs);
+    } else {
+        a.p.ad = adjoint_set(b.bwd_copy[rd ^ 1], b.cells);
+        a.in_ad = adjoint_set(b.bwd_copy[rd], b.cells);
+    }
+    a.items = b.ditems.p + (backward ? b.items[0].size() : 0);
+    a.rsrc = b.rsrc.p;
+    a.rsp = b.rsp;
+    a.fx = b.fx;
+    a.fz = b.fz;
+    a.one = 1.f;
+    return a;
+}
+// the reconstruction (and the adjoint) as the backward steps find them
+void start_backward(sfwi_handle *h) {
+    Batch &b = h->b;
+    if (h->snap_every > 0 || !(b.bwd_pairs || b.way[0])) return;
+    PairStart s{};
+    for (int c = 0; c < 2; c++) {
+        s.src[c] = b.way[0] ? b.fwd_copy[c] : b.grid.p;
+        s.dst[c] = b.bwd_pairs ? b.bwd_copy[c] : b.grid.p;
+    }
+    s.from_pairs = b.fwd_pairs;
+    s.to_pairs = b.bwd_pairs;
+    s.P = b.P;
+    s.cells = b.cells;
+    s.geo = b.dgeo.p;
+    s.aux = b.daux.p;
+    launch_pair_start(s, b.max_nxpml, b.nshots, h->st);
+    h->launches++;
+}
+int march_count(const Batch &b, int it, bool backward) {
+    const std::vector<int> &act = b.items_active[backward];
+    return act.empty() ? (int)b.items[backward].size() : act[it];
+}
+
 int build_batch(sfwi_handle *h, const std::vector<ShotIn> &shots) {
     Batch &b = h->b;
     const int pml = h->pml, nt = h->nt;
@@ -855,6 +1187,7 @@ int upload_batch(sfwi_handle *h, const std::vector<ShotIn> &shots, bool forward_
     // zero the state (fields, memory variables, accumulators) and the records
     CK(cudaMemsetAsync(b.grid.p, 0, (size_t)NSTATE * b.cells * sizeof(float), st));
     CK(cudaMemsetAsync(b.recs.p, 0, recs * sizeof(float), st));
+    if (int rc = upload_march(h, forward_only)) return rc;
     // observed records, trace-major ([ntr][its nt] on the host; a shot with
     // fewer steps than the batch keeps zeros after its last sample), copied
     // on the records stream after the zeroing above; the run's stream waits
@@ -922,6 +1255,10 @@ int upload_batch(sfwi_handle *h, const std::vector<ShotIn> &shots, bool forward_
     CK(cudaEventRecord(h->ev[4], st));
     launch_setup(a, b.nshots, b.max_nxpml, st);
     h->launches++;
+    if (b.way[0] || b.way[1]) {
+        launch_march_factors(MarchFactors{b.g(C_DX), b.g(C_DZ), h->dt, b.cells, b.fx, b.fz}, st);
+        h->launches++;
+    }
     CK(cudaGetLastError());
     return SFWI_OK;
 }
@@ -957,7 +1294,11 @@ std::vector<long long> shape_signature(sfwi_handle *h, bool forward_only) {
                                 (long long)(uintptr_t)b.lr.p, (long long)(uintptr_t)b.rrow.p,
                                 (long long)(uintptr_t)b.rsrc.p, (long long)(uintptr_t)b.dtiles.p,
                                 (long long)(uintptr_t)b.dgeo.p, (long long)(uintptr_t)h->sou.p, b.strip_steps,
-                                b.strip_chunk, (long long)(uintptr_t)h->htb.p, (long long)(uintptr_t)h->hlr.p};
+                                b.strip_chunk, (long long)(uintptr_t)h->htb.p, (long long)(uintptr_t)h->hlr.p,
+                                (long long)(uintptr_t)b.way[0], (long long)(uintptr_t)b.way[1],
+                                (long long)(uintptr_t)b.grid2.p,
+                                (long long)(uintptr_t)b.ditems.p, (long long)b.items[0].size(),
+                                (long long)b.items[1].size(), b.max_nxpml};
     for (auto &t : b.tiles) s.push_back(((long long)t.shot << 40) ^ ((long long)t.x0 << 24) ^ (t.z0 << 8) ^ t.flags);
     for (auto &g : b.geo) {
         s.push_back(g.isx * 100003LL + g.isz);
@@ -1005,13 +1346,22 @@ int strip_copy(sfwi_handle *h, int chunk, bool to_host) {
 // for the first backward steps).
 int enqueue_forward(sfwi_handle *h, const Params &p, bool forward_only) {
     const bool born = h->stage == 2;
-    (void)forward_only;
-    const int n = h->b.strip_chunk, nc = h->b.strip_chunks;
+    Batch &b = h->b;
+    const int n = b.strip_chunk, nc = b.strip_chunks;
     for (int it = 0; it < h->nt; it++) {
         if (n && it % n == 0 && it / n >= 2) CK(cudaStreamWaitEvent(h->st, h->ev_copy[(it / n) % 2], 0));
-        const Params q = step_params(h, p, it);
-        h->tv->launch(0, q, h->b.tm, it, born, 1.f, h->st);
-        h->tv->launch(1, q, h->b.tm, it, born, 1.f, h->st);
+        if (b.way[0]) {
+            // steps read one copy of the fields and write the other; a
+            // modelling run ends in the first one
+            const int rd = (it + (forward_only ? h->nt : 0)) & 1;
+            const MarchArgs a = march_args(h, p, rd, false);
+            b.way[0]->fwd(a, b.mf[rd], march_count(b, it, false), it, born, h->st);
+            if (p.snap && it % p.snap_every == 0) launch_snap_store(a, b.max_nxpml, it, b.fwd_pairs, h->st);
+        } else {
+            const Params q = step_params(h, p, it);
+            h->tv->launch(0, q, b.tm, it, born, 1.f, h->st);
+            h->tv->launch(1, q, b.tm, it, born, 1.f, h->st);
+        }
         if (n && (it + 1) % n == 0 && (it + 1) / n <= nc - 2)
             if (int rc = strip_copy(h, it / n, true)) return rc;
     }
@@ -1023,13 +1373,25 @@ int enqueue_forward(sfwi_handle *h, const Params &p, bool forward_only) {
 // which starts once chunk c + 2, the slot's last user, is done.
 int enqueue_backward(sfwi_handle *h, const Params &p) {
     const float adj = h->stage == 1 ? 1.f : -1.f;
-    const int n = h->b.strip_chunk, nc = h->b.strip_chunks;
+    Batch &b = h->b;
+    const int n = b.strip_chunk, nc = b.strip_chunks;
+    int max_nzpml = 0;
+    for (const ShotGeo &g : b.geo) max_nzpml = std::max(max_nzpml, g.nzpml);
     for (int it = h->nt - 1; it >= 0; it--) {
         const int c = n ? it / n : 0;
         if (n && (it + 1) % n == 0 && c <= nc - 3) CK(cudaStreamWaitEvent(h->st, h->ev_copy[c % 2], 0));
-        const Params q = step_params(h, p, it);
-        h->tv->launch(2, q, h->b.tm, it, false, adj, h->st);
-        h->tv->launch(3, q, h->b.tm, it, false, adj, h->st);
+        if (b.way[1]) {
+            // (a shot's forward steps end in copy nt & 1, whatever the run's length)
+            const int rd = (it + 1) & 1;
+            const MarchArgs a = march_args(h, p, rd, true);
+            b.way[1]->bwd(a, b.mb[rd], march_count(b, it, true), it, adj, h->st);
+            if (p.snap && it % p.snap_every == 0)
+                launch_snap_image(a, b.max_nxpml - 2 * h->pml, max_nzpml - 2 * h->pml, it, h->st);
+        } else {
+            const Params q = step_params(h, p, it);
+            h->tv->launch(2, q, b.tm, it, false, adj, h->st);
+            h->tv->launch(3, q, b.tm, it, false, adj, h->st);
+        }
         if (n && it % n == 0 && c >= 2)
             if (int rc = strip_copy(h, c - 2, false)) return rc;
     }
@@ -1124,7 +1486,15 @@ int run_batch(sfwi_handle *h, const std::vector<ShotIn> &shots, int mode, double
     if (!h->b.tlen.empty() && ((mode != RUN_FORWARD && misfit_kind != SFWI_MISFIT_L2) || h->snap_every > 0))
         return fail(SFWI_E_ARG, "shots of different lengths in one run take the L2 misfit and no snapshots");
     ObservedGuard obs_guard{h};
+    plan_march(h, forward_only);
     rc = upload_batch(h, shots, forward_only, mode != RUN_FORWARD);
+    if (rc == SFWI_E_NOMEM && h->b.grid2.p) {
+        // an earlier run's copy of the fields may hold what this one needs
+        CK(cudaStreamSynchronize(h->st));
+        h->b.grid2.release();
+        no_march(h->b);
+        rc = upload_batch(h, shots, forward_only, mode != RUN_FORWARD);
+    }
     if (rc) return rc;
     Batch &b = h->b;
     b.ready = true;
@@ -1148,7 +1518,8 @@ int run_batch(sfwi_handle *h, const std::vector<ShotIn> &shots, int mode, double
         CK(cudaGraphLaunch(b.gfwd, st));
     else if ((rc = enqueue_forward(h, p, forward_only)))
         return rc;
-    h->launches += 2LL * nt;
+    const long long snaps = p.snap ? b.nsnap : 0;
+    h->launches += b.way[0] ? nt + snaps : 2LL * nt;
     CK(cudaGetLastError());
     CK(cudaEventRecord(h->ev[1], st));
     // receiver-row records to trace-major records
@@ -1216,11 +1587,12 @@ int run_batch(sfwi_handle *h, const std::vector<ShotIn> &shots, int mode, double
     CK(cudaGetLastError());
     nvtxMarkA("sfwi backward sweeps");
     CK(cudaEventRecord(h->ev[2], st));
+    start_backward(h);
     if (h->use_graphs)
         CK(cudaGraphLaunch(b.gbwd, st));
     else if ((rc = enqueue_backward(h, p)))
         return rc;
-    h->launches += 2LL * nt;
+    h->launches += b.way[1] ? nt + snaps : 2LL * nt;
     CK(cudaGetLastError());
     CK(cudaEventRecord(h->ev[3], st));
     FinalArgs fa{};
@@ -1277,7 +1649,7 @@ template <class F>
 void for_each_buf(sfwi_handle *h, F f) {
     Batch &b = h->b;
     f(b.grid), f(b.tb), f(b.lr), f(b.rrow), f(b.rsrc), f(b.recs), f(b.tmis), f(b.dsigma), f(b.dgeo), f(b.dtiles);
-    f(b.dtrow), f(b.drtr), f(b.derr), f(b.dctr), f(b.snap), f(b.sscale), f(b.otscr);
+    f(b.grid2), f(b.ditems), f(b.dtrow), f(b.drtr), f(b.derr), f(b.dctr), f(b.snap), f(b.sscale), f(b.otscr);
     f(h->sou), f(h->vp_all), f(h->vs_all), f(h->rho_all), f(h->dvp_all), f(h->dvs_all);
     f(h->gpp), f(h->gps), f(h->gil), f(h->grh), f(h->ls_buf);
     f(h->mvp), f(h->mvs), f(h->mrho), f(h->mdvp), f(h->mdvs), f(h->mgrad);
@@ -1443,6 +1815,7 @@ int born_adjoint(sfwi_handle *h, const std::vector<ShotIn> &q, double *img_vp, d
     h->b.ready = false;
     h->last_perm.clear();
     if (int rc = build_batch(h, q)) return rc;
+    no_march(h->b);
     ObservedGuard obs_guard{h};
     if (int rc = upload_batch(h, q, false, true)) return rc;
     Batch &b = h->b;
@@ -1699,6 +2072,8 @@ int sfwi_create(sfwi_handle **out, int stage, const float *sou, float dx, float 
         cudaError_t e = cudaSuccess;
         h->tv = tile_variant(SFWI_TILE_16x32);
         for (int v = 0; v < SFWI_NUM_TILE_SHAPES && e == cudaSuccess; v++) e = tile_variant(v)->configure();
+        for (const MarchVariant *m : {march_wide(), march_burst()})
+            if (e == cudaSuccess) e = m->configure();
         if (e != cudaSuccess) {
             rc = fail(SFWI_E_CUDA, "kernel attributes: %s", cudaGetErrorString(e));
             break;
@@ -2234,6 +2609,13 @@ int sfwi_autotune(sfwi_handle *h, int reps, int *choice, float *out_ms) {
     // accumulators, which the next run clears
     float best = 0.f;
     int pick = 0;
+    // the shapes are the sweeps'; whether a batch runs whole steps per launch
+    // stays a matter of its size
+    struct KeepMarch {
+        sfwi_handle *h;
+        bool ok;
+        ~KeepMarch() { h->march_ok = ok; }
+    } keep{h, h->march_ok};
     for (int v = 0; v < SFWI_NUM_TILE_SHAPES; v++) {
         if (int rc = sfwi_set_tile_shape(h, v)) return rc;
         float ms[4];
@@ -2280,6 +2662,35 @@ int sfwi_debug_read_grid(sfwi_handle *h, int array, float *dst) {
     Batch &b = h->b;
     if (!b.ready) return fail(SFWI_E_STATE, "no batch on the device");
     CK(cudaSetDevice(h->device));
+    // after whole steps per launch the fields lie in their own layout
+    // (layout_march); the last step wrote the first copy.  The backward steps
+    // keep no scattered field.
+    if ((b.way[0] || b.way[1]) && array < G_LAM) {
+        const bool back = !h->last_forward_only;
+        if (array >= SC_VX && array < AD_VX && back && h->stage == 2 && b.bwd_pairs) {
+            std::memset(dst, 0, b.cells * sizeof(float));
+            return SFWI_OK;
+        }
+        const float *src = nullptr;
+        size_t stride = 2;
+        const int copy = back ? h->nt & 1 : 0;  // where the forward steps ended
+        if (back && b.bwd_pairs && (array < SC_VX || array >= AD_VX)) {
+            // reconstruction, adjoint
+            const int k = array < SC_VX ? array : array == AD_MTXZ ? BG_MTXZ : array - AD_VX;
+            src = b.bwd_copy[0] + 2 * (size_t)k * b.cells + (array >= AD_VX);
+        } else if (b.fwd_pairs && array < AD_VX && !(back && array < SC_VX && h->snap_every == 0)) {
+            src = b.fwd_copy[copy] + 2 * (size_t)(array % SC_VX) * b.cells + (array >= SC_VX);
+        } else if (b.way[0] && array < SC_VX && h->snap_every > 0) {
+            src = b.fwd_copy[copy] + (size_t)array * b.cells;
+            stride = 1;
+        }
+        if (src) {
+            CK(cudaMemcpy2DAsync(dst, sizeof(float), src, stride * sizeof(float), sizeof(float), b.cells,
+                                 cudaMemcpyDeviceToHost, h->st));
+            CK(cudaStreamSynchronize(h->st));
+            return SFWI_OK;
+        }
+    }
     CK(cudaMemcpyAsync(dst, b.g(array), b.cells * sizeof(float), cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));
     return SFWI_OK;
@@ -2331,6 +2742,7 @@ int sfwi_set_tile_shape(sfwi_handle *h, int shape) {
     if (int rc = check(h)) return rc;
     if (shape < 0 || shape >= SFWI_NUM_TILE_SHAPES) return fail(SFWI_E_ARG, "tile shape %d out of range", shape);
     h->tile_auto = false;
+    h->march_ok = false;  // the shape is the sweeps'
     if (h->tv == tile_variant(shape)) return SFWI_OK;
     h->tv = tile_variant(shape);
     Batch &b = h->b;

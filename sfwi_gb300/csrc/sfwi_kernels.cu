@@ -54,7 +54,9 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include "sfwi_cell.cuh"
 #include "sfwi_launch.h"
+#include "sfwi_pipe.cuh"
 
 #ifndef SFWI_VARIANT_NS
 #define SFWI_VARIANT_NS v16x32
@@ -63,12 +65,6 @@
 
 namespace sfwi {
 namespace SFWI_VARIANT_NS {
-
-// 8th-order staggered first-derivative weights, sfwi-stage1/FD2DGPU.cuh:16
-constexpr float K1 = (float)(1225.0 / 1024.0);
-constexpr float K2 = (float)(-245.0 / 3072.0);
-constexpr float K3 = (float)(49.0 / 5120.0);
-constexpr float K4 = (float)(-5.0 / 7168.0);
 
 #ifndef SFWI_STAGES
 #define SFWI_STAGES 2
@@ -99,41 +95,8 @@ constexpr int CORE = TX * TZ;  // floats of a core tile
 constexpr uint32_t BOX_BYTES = BOX * 4u, CORE_BYTES = CORE * 4u;
 
 // ----------------------------------------------------------------------------
-// TMA / mbarrier primitives
+// barriers of the consumer threads
 // ----------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
-// Programmatic dependent launch: the step kernels are launched so that the
-// next one may start while this one drains.  griddep_wait blocks until the
-// previous kernel of the stream has completed and its writes are visible
-// (at once when there is no such kernel); every read of data another kernel
-// wrote, and every write, comes after it.  griddep_launch lets the next
-// kernel's CTAs be scheduled onto SMs this kernel's CTAs leave.
-__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 // barrier 1 over the NTHREADS consumer threads (the producer warp is not in it)
 __device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, %0;" ::"n"(NTHREADS) : "memory"); }
 __device__ __forceinline__ bool consumer_any(bool v) {
@@ -148,31 +111,6 @@ __device__ __forceinline__ bool consumer_any(bool v) {
         : "memory");
     return r != 0;
 }
-// bounded wait: false when the phase did not complete within `limit` tries
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint32_t limit) {
-    for (uint32_t i = 0; i < limit; i++)
-        if (mbar_try_wait(bar, parity)) return true;
-    return false;
-}
-// 3-D tiled bulk tensor load global -> shared, completion counted on `bar`
-__device__ __forceinline__ void tma_load(float *dst, const CUtensorMap *map, int col, int row, int arr,
-                                         uint64_t *bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
-        "[%5];" ::"r"(smem_u32(dst)),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(col), "r"(row), "r"(arr), "r"(smem_u32(bar))
-        : "memory");
-}
-
-// 2-D tiled bulk tensor load global -> shared (x = innermost coordinate)
-__device__ __forceinline__ void tma_load_2d(float *dst, const CUtensorMap *map, int x, int y, uint64_t *bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], "
-        "[%4];" ::"r"(smem_u32(dst)),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar))
-        : "memory");
-}
-
 // ----------------------------------------------------------------------------
 // stencils on staged boxes (row pitch BZ)
 // ----------------------------------------------------------------------------
@@ -267,11 +205,6 @@ __device__ __forceinline__ WC loadw(const float *f, int r, int c) {
     return o;
 }
 __device__ __forceinline__ float2 pr(const WC &s, int i) { return make_float2(s.w[i], s.w[i + 1]); }
-// k*(p - q) + a on a pair
-__device__ __forceinline__ float2 kdiff2(float k, float2 p, float2 q, float2 a) {
-    const float2 d = __ffma2_rn(q, make_float2(-1.f, -1.f), p);
-    return __ffma2_rn(make_float2(k, k), d, a);
-}
 // D+z: sum_k K_k (f[c+k] - f[c-k+1]) on the cell pairs as FP32x2
 __device__ __forceinline__ VC dzp(const WC &s) {
     VC a;
@@ -360,23 +293,15 @@ __device__ __forceinline__ CellMap cell_map(const Params &p, const Tile &t, cons
 
 __device__ __forceinline__ void core4(const float *core, int slot, int ci, float o[CPT]) { ldc(core + slot * CORE + ci, o); }
 
-// PML factors of a frame cell: the split update (d1*m + c*D)/d2 is evaluated
-// as (d1*m + c*D) * (1/d2) with a correctly rounded reciprocal, one rounding
-// more than a division
+// PML factors of this thread's cells
 struct Damp {
-    float d1[CPT], r2[CPT], d3[CPT], r4[CPT];
+    Damp2 p[NP];
 };
 __device__ __forceinline__ Damp make_damp(const Params &p, const float x[CPT], const float z[CPT]) {
     Damp d;
 #pragma unroll
-    for (int j = 0; j < CPT; j++) {
-        // 1 -+ (dt d)/2: halving is exact, so one fused step rounds once
-        const float tx = p.dt * x[j], tz = p.dt * z[j];
-        d.d1[j] = fmaf(tx, -0.5f, 1.f);
-        d.r2[j] = __frcp_rn(fmaf(tx, 0.5f, 1.f));
-        d.d3[j] = fmaf(tz, -0.5f, 1.f);
-        d.r4[j] = __frcp_rn(fmaf(tz, 0.5f, 1.f));
-    }
+    for (int h = 0; h < NP; h++)
+        d.p[h] = make_damp2(p.dt, make_float2(x[2 * h], x[2 * h + 1]), make_float2(z[2 * h], z[2 * h + 1]));
     return d;
 }
 
@@ -389,11 +314,10 @@ struct SState {
 
 // FP32x2 helpers on the cells (2h, 2h+1) of a four-cell group
 __device__ __forceinline__ float2 P2(const float v[CPT], int h) { return make_float2(v[2 * h], v[2 * h + 1]); }
-__device__ __forceinline__ void S2(float v[CPT], int h, float2 x) {
+__device__ __forceinline__ void W2(float v[CPT], int h, float2 x) {
     v[2 * h] = x.x;
     v[2 * h + 1] = x.y;
 }
-__device__ __forceinline__ float2 B2(float x) { return make_float2(x, x); }
 // store a packed pair into cells 2h, 2h+1 of v where the cell is updated
 __device__ __forceinline__ void sel2(float v[CPT], int h, float2 x, const bool ok[CPT]) {
     if (ok[2 * h]) v[2 * h] = x.x;
@@ -405,10 +329,6 @@ __device__ __forceinline__ void pick2(float v[CPT], int h, float2 split, float2 
     if (m.ok[2 * h]) v[2 * h] = m.split[2 * h] ? split.x : plain.x;
     if (m.ok[2 * h + 1]) v[2 * h + 1] = m.split[2 * h + 1] ? split.y : plain.y;
 }
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-
 // velocity update of one field set on this thread's four cells:
 //   vx += dir*ib*(dtdx*ax + dtdz*bz),  vz += dir*ib*(dtdx*dx_ + dtdz*cz)
 // with the split form in frame cells; stores the new state.
@@ -416,48 +336,32 @@ template <bool FRAME>
 __device__ __forceinline__ void v_apply(const Params &p, const CellMap &m, const FieldSet &f, VState &s,
                                         const float ib[CPT], const Damp &d, float dir, const VC &ax, const VC &bz,
                                         const VC &dx_, const VC &cz) {
-    if (!FRAME) {
-        // tile without PML cells: all four cells are updated (FP32x2)
-        const float2 tx = B2(dir * p.dtdx), tz = B2(dir * p.dtdz);
+    const float2 tx = B2(dir * p.dtdx), tz = B2(dir * p.dtdz);
 #pragma unroll
-        for (int h = 0; h < NP; h++) {
-            const float2 i2 = P2(ib, h);
-            const float2 cx = mul2(i2, tx), cz2 = mul2(i2, tz);
-            S2(s.vx, h, add2(P2(s.vx, h), fma2(cx, P2(ax.v, h), mul2(cz2, P2(bz.v, h)))));
-            S2(s.vz, h, add2(P2(s.vz, h), fma2(cx, P2(dx_.v, h), mul2(cz2, P2(cz.v, h)))));
-        }
-        stc(f.vx + m.gi, s.vx);
-        stc(f.vz + m.gi, s.vz);
-        return;
-    }
-    // tile with PML cells: the split update of the reference in damped cells,
-    //   v_x = (d1 v_x + c_x D_x) r2,  v_z = (d3 v_z + c_z D_z) r4,  v = v_x + v_z,
-    // with the x-part kept in mx and the z-part = v - mx; the plain update
-    // above in the tile's other cells; cells outside the update region keep
-    // their values
-    {
-        const float2 tx = B2(dir * p.dtdx), tz = B2(dir * p.dtdz), neg = B2(-1.f);
-#pragma unroll
-        for (int h = 0; h < NP; h++) {
-            const float2 i2 = P2(ib, h);
-            const float2 cx = mul2(i2, tx), cz2 = mul2(i2, tz);
-            const float2 px = add2(P2(s.vx, h), fma2(cx, P2(ax.v, h), mul2(cz2, P2(bz.v, h))));
-            const float2 pz = add2(P2(s.vz, h), fma2(cx, P2(dx_.v, h), mul2(cz2, P2(cz.v, h))));
-            const float2 d1 = P2(d.d1, h), r2 = P2(d.r2, h), d3 = P2(d.d3, h), r4 = P2(d.r4, h);
-            const float2 mx = P2(s.mx, h), mz = P2(s.mz, h);
-            const float2 xx = mul2(fma2(d1, mx, mul2(cx, P2(ax.v, h))), r2);
-            const float2 xz = mul2(fma2(d3, fma2(mx, neg, P2(s.vx, h)), mul2(cz2, P2(bz.v, h))), r4);
-            const float2 zx = mul2(fma2(d1, mz, mul2(cx, P2(dx_.v, h))), r2);
-            const float2 zz = mul2(fma2(d3, fma2(mz, neg, P2(s.vz, h)), mul2(cz2, P2(cz.v, h))), r4);
-            sel2(s.mx, h, xx, m.split);
-            sel2(s.mz, h, zx, m.split);
-            pick2(s.vx, h, add2(xx, xz), px, m);
-            pick2(s.vz, h, add2(zx, zz), pz, m);
+    for (int h = 0; h < NP; h++) {
+        const float2 i2 = P2(ib, h);
+        const float2 cx = mul2(i2, tx), cz2 = mul2(i2, tz);
+        const V2 old{P2(s.vx, h), P2(s.vz, h)};
+        const V2 pl = v_plain2(old, cx, cz2, P2(ax.v, h), P2(bz.v, h), P2(dx_.v, h), P2(cz.v, h));
+        if (!FRAME) {
+            // tile without PML cells: all of the thread's cells are updated
+            W2(s.vx, h, pl.x);
+            W2(s.vz, h, pl.z);
+        } else {
+            // tile with PML cells: the split update in damped cells (x-parts
+            // in mx, mz), the plain one in the tile's other cells; cells
+            // outside the update region keep their values
+            V2 xp{P2(s.mx, h), P2(s.mz, h)};
+            const V2 sp = v_split2(old, xp, d.p[h], cx, cz2, P2(ax.v, h), P2(bz.v, h), P2(dx_.v, h), P2(cz.v, h));
+            sel2(s.mx, h, xp.x, m.split);
+            sel2(s.mz, h, xp.z, m.split);
+            pick2(s.vx, h, sp.x, pl.x, m);
+            pick2(s.vz, h, sp.z, pl.z, m);
         }
     }
     stc(f.vx + m.gi, s.vx);
     stc(f.vz + m.gi, s.vz);
-    if (m.any_split) {
+    if (FRAME && m.any_split) {
         stc(f.mvx + m.gi, s.mx);
         stc(f.mvz + m.gi, s.mz);
     }
@@ -465,86 +369,41 @@ __device__ __forceinline__ void v_apply(const Params &p, const CellMap &m, const
 
 // stress update of one field set from velocity derivatives
 //   a = D-x vx, b = D-z vz, c = D+z vx, d = D+x vz
-// with optional Born terms added to the split parts first (born != nullptr).
-template <bool FRAME>
+// with the Born increments of the split parts (BORN: one Born2 per pair).
+template <bool FRAME, bool BORN>
 __device__ __forceinline__ void s_apply(const Params &p, const CellMap &m, const FieldSet &f, SState &s,
                                         const float lam[CPT], const float mu[CPT], const Damp &dm, float dir, const VC &a,
-                                        const VC &b, const VC &c, const VC &d, const float (*born)[CPT]) {
-    if (!FRAME) {
-        // tile without PML cells: all four cells are updated (FP32x2)
-        const float2 tx = B2(dir * p.dtdx), tz = B2(dir * p.dtdz);
+                                        const VC &b, const VC &c, const VC &d, const Born2 *born) {
+    const float2 tx = B2(dir * p.dtdx), tz = B2(dir * p.dtdz);
 #pragma unroll
-        for (int h = 0; h < NP; h++) {
-            const float2 l = P2(lam, h), u = P2(mu, h);
-            const float2 l2m = fma2(u, B2(2.f), l);
-            const float2 ax = mul2(tx, P2(a.v, h)), bz = mul2(tz, P2(b.v, h));
-            const float2 cz = mul2(tz, P2(c.v, h)), dx_ = mul2(tx, P2(d.v, h));
-            float2 xx = P2(s.xx, h), zz = P2(s.zz, h), xz = P2(s.xz, h);
-            if (born) {
-                xx = add2(xx, add2(P2(born[0], h), P2(born[1], h)));
-                zz = add2(zz, add2(P2(born[2], h), P2(born[3], h)));
-                xz = add2(xz, add2(P2(born[4], h), P2(born[5], h)));
-            }
-            S2(s.xx, h, add2(xx, fma2(l2m, ax, mul2(l, bz))));
-            S2(s.zz, h, add2(zz, fma2(l, ax, mul2(l2m, bz))));
-            S2(s.xz, h, fma2(u, fma2(tz, P2(c.v, h), dx_), xz));
-        }
-        stc(f.txx + m.gi, s.xx);
-        stc(f.tzz + m.gi, s.zz);
-        stc(f.txz + m.gi, s.xz);
-        return;
-    }
-    // tile with PML cells: the split updates of the reference in damped cells
-    // (x-parts in mxx, mzz, mxz; z-part = total - x-part), Born increments
-    // added to the split parts before the damping; the plain update above in
-    // the tile's other cells
-    {
-        const float2 tx = B2(dir * p.dtdx), tz = B2(dir * p.dtdz), neg = B2(-1.f);
-#pragma unroll
-        for (int h = 0; h < NP; h++) {
-            const float2 l = P2(lam, h), u = P2(mu, h);
-            const float2 l2m = fma2(u, B2(2.f), l);
-            const float2 ax = mul2(tx, P2(a.v, h)), bz = mul2(tz, P2(b.v, h));
-            const float2 cz = mul2(tz, P2(c.v, h)), dx_ = mul2(tx, P2(d.v, h));
-            float2 pxx = P2(s.xx, h), pzz = P2(s.zz, h), pxz = P2(s.xz, h);
-            if (born) {
-                pxx = add2(pxx, add2(P2(born[0], h), P2(born[1], h)));
-                pzz = add2(pzz, add2(P2(born[2], h), P2(born[3], h)));
-                pxz = add2(pxz, add2(P2(born[4], h), P2(born[5], h)));
-            }
-            pxx = add2(pxx, fma2(l2m, ax, mul2(l, bz)));
-            pzz = add2(pzz, fma2(l, ax, mul2(l2m, bz)));
-            pxz = fma2(u, fma2(tz, P2(c.v, h), dx_), pxz);
-            const float2 d1 = P2(dm.d1, h), r2 = P2(dm.r2, h), d3 = P2(dm.d3, h), r4 = P2(dm.r4, h);
-            float2 mxx = P2(s.mxx, h), mzz = P2(s.mzz, h), mxz = P2(s.mxz, h);
-            float2 zxx = fma2(mxx, neg, P2(s.xx, h)), zzz = fma2(mzz, neg, P2(s.zz, h));
-            float2 zxz = fma2(mxz, neg, P2(s.xz, h));
-            if (born) {
-                mxx = add2(mxx, P2(born[0], h));
-                zxx = add2(zxx, P2(born[1], h));
-                mzz = add2(mzz, P2(born[2], h));
-                zzz = add2(zzz, P2(born[3], h));
-                mxz = add2(mxz, P2(born[4], h));
-                zxz = add2(zxz, P2(born[5], h));
-            }
-            const float2 nxx_x = mul2(fma2(d1, mxx, mul2(l2m, ax)), r2);
-            const float2 nxx_z = mul2(fma2(d3, zxx, mul2(l, bz)), r4);
-            const float2 nzz_x = mul2(fma2(d1, mzz, mul2(l, ax)), r2);
-            const float2 nzz_z = mul2(fma2(d3, zzz, mul2(l2m, bz)), r4);
-            const float2 nxz_x = mul2(fma2(d1, mxz, mul2(u, dx_)), r2);
-            const float2 nxz_z = mul2(fma2(d3, zxz, mul2(u, cz)), r4);
-            sel2(s.mxx, h, nxx_x, m.split);
-            sel2(s.mzz, h, nzz_x, m.split);
-            sel2(s.mxz, h, nxz_x, m.split);
-            pick2(s.xx, h, add2(nxx_x, nxx_z), pxx, m);
-            pick2(s.zz, h, add2(nzz_x, nzz_z), pzz, m);
-            pick2(s.xz, h, add2(nxz_x, nxz_z), pxz, m);
+    for (int h = 0; h < NP; h++) {
+        const float2 l = P2(lam, h), u = P2(mu, h);
+        const S2 old{P2(s.xx, h), P2(s.zz, h), P2(s.xz, h)};
+        const Born2 q = BORN ? born[h] : Born2{};
+        const S2 pl = s_plain2<BORN>(old, tx, tz, l, u, P2(a.v, h), P2(b.v, h), P2(c.v, h), P2(d.v, h), q);
+        if (!FRAME) {
+            // tile without PML cells: all of the thread's cells are updated
+            W2(s.xx, h, pl.xx);
+            W2(s.zz, h, pl.zz);
+            W2(s.xz, h, pl.xz);
+        } else {
+            // tile with PML cells: the split updates in damped cells
+            // (x-parts in mxx, mzz, mxz), the plain one in the other cells
+            S2 xp{P2(s.mxx, h), P2(s.mzz, h), P2(s.mxz, h)};
+            const S2 sp = s_split2<BORN>(old, xp, dm.p[h], tx, tz, l, u, P2(a.v, h), P2(b.v, h), P2(c.v, h),
+                                         P2(d.v, h), q);
+            sel2(s.mxx, h, xp.xx, m.split);
+            sel2(s.mzz, h, xp.zz, m.split);
+            sel2(s.mxz, h, xp.xz, m.split);
+            pick2(s.xx, h, sp.xx, pl.xx, m);
+            pick2(s.zz, h, sp.zz, pl.zz, m);
+            pick2(s.xz, h, sp.xz, pl.xz, m);
         }
     }
     stc(f.txx + m.gi, s.xx);
     stc(f.tzz + m.gi, s.zz);
     stc(f.txz + m.gi, s.xz);
-    if (m.any_split) {
+    if (FRAME && m.any_split) {
         stc(f.mtxx + m.gi, s.mxx);
         stc(f.mtzz + m.gi, s.mzz);
         stc(f.mtxz + m.gi, s.mxz);
@@ -1034,32 +893,20 @@ __global__ void __launch_bounds__(BLOCK_THREADS, CTAS_PER_SM)
         Damp dm{};
         if (frame) dm = make_damp(p, ex, ez);
         if (frame)
-            s_apply<true>(p, m, p.bg, bg, lam, mu, dm, 1.f, a, b, cc, d, nullptr);
+            s_apply<true, false>(p, m, p.bg, bg, lam, mu, dm, 1.f, a, b, cc, d, nullptr);
         else
-            s_apply<false>(p, m, p.bg, bg, lam, mu, dm, 1.f, a, b, cc, d, nullptr);
+            s_apply<false, false>(p, m, p.bg, bg, lam, mu, dm, 1.f, a, b, cc, d, nullptr);
         if (BORN) {
             // Born virtual source from the updated background velocity
-            // (add_born_source_components, sfwi-stage2/born.cu:788-798); bp/bs
-            // are zero outside the Born region
-            float born[6][CPT];
+            Born2 born[NP];
 #pragma unroll
-            for (int h = 0; h < NP; h++) {
-                const float2 bp2 = P2(bp, h), bs2 = P2(bs, h);
-                const float2 mix = fma2(bs2, B2(-2.f), bp2);
-                const float2 ax = mul2(P2(a.v, h), B2(p.idx)), bz = mul2(P2(b.v, h), B2(p.idz));
-                const float2 dx_ = mul2(P2(d.v, h), B2(p.idx)), cz = mul2(P2(cc.v, h), B2(p.idz));
-                const float2 dt2 = B2(p.dt);
-                S2(born[0], h, mul2(dt2, mul2(bp2, ax)));
-                S2(born[1], h, mul2(dt2, mul2(mix, bz)));
-                S2(born[2], h, mul2(dt2, mul2(mix, ax)));
-                S2(born[3], h, mul2(dt2, mul2(bp2, bz)));
-                S2(born[4], h, mul2(dt2, mul2(bs2, dx_)));
-                S2(born[5], h, mul2(dt2, mul2(bs2, cz)));
-            }
+            for (int h = 0; h < NP; h++)
+                born[h] = born2(P2(bp, h), P2(bs, h), p.idx, p.idz, p.dt, P2(a.v, h), P2(b.v, h), P2(cc.v, h),
+                                P2(d.v, h));
             if (frame)
-                s_apply<true>(p, m, p.sc, sc, lam, mu, dm, 1.f, as, bs_, cs, ds, born);
+                s_apply<true, true>(p, m, p.sc, sc, lam, mu, dm, 1.f, as, bs_, cs, ds, born);
             else
-                s_apply<false>(p, m, p.sc, sc, lam, mu, dm, 1.f, as, bs_, cs, ds, born);
+                s_apply<false, true>(p, m, p.sc, sc, lam, mu, dm, 1.f, as, bs_, cs, ds, born);
         }
     };
     if (SNAP && snap_step(p, it) && p.snap_fmt != SNAP_F32) {
@@ -1077,32 +924,24 @@ __global__ void __launch_bounds__(BLOCK_THREADS, CTAS_PER_SM)
 __device__ __forceinline__ void adjoint_stress(const Params &p, const CellMap &m, bool frame, const Damp &dm,
                                                float adj_dir, const VC &aa, const VC &ba, const VC &ca, const VC &da,
                                                float axx[CPT], float azz[CPT], float axz[CPT], float amxz[CPT]) {
-    if (!frame) {
-        const float2 tx = B2(adj_dir * p.dtdx), tz = B2(adj_dir * p.dtdz);
+    const float2 tx = B2(adj_dir * p.dtdx), tz = B2(adj_dir * p.dtdz);
 #pragma unroll
-        for (int h = 0; h < NP; h++) {
-            S2(axx, h, fma2(tx, P2(aa.v, h), P2(axx, h)));
-            S2(azz, h, fma2(tz, P2(ba.v, h), P2(azz, h)));
-            S2(axz, h, add2(P2(axz, h), fma2(tx, P2(da.v, h), mul2(tz, P2(ca.v, h)))));
-        }
-    } else {
-        // tile with PML cells: the split update in damped cells, the plain
-        // one above in the others
-        const float2 tx = B2(adj_dir * p.dtdx), tz = B2(adj_dir * p.dtdz), neg = B2(-1.f);
-#pragma unroll
-        for (int h = 0; h < NP; h++) {
-            const float2 pxx = fma2(tx, P2(aa.v, h), P2(axx, h));
-            const float2 pzz = fma2(tz, P2(ba.v, h), P2(azz, h));
-            const float2 pxz = add2(P2(axz, h), fma2(tx, P2(da.v, h), mul2(tz, P2(ca.v, h))));
-            const float2 d1 = P2(dm.d1, h), r2 = P2(dm.r2, h), d3 = P2(dm.d3, h), r4 = P2(dm.r4, h);
-            const float2 nxx = mul2(fma2(d1, P2(axx, h), mul2(tx, P2(aa.v, h))), r2);
-            const float2 nzz = mul2(fma2(d3, P2(azz, h), mul2(tz, P2(ba.v, h))), r4);
-            const float2 nx_ = mul2(fma2(d1, P2(amxz, h), mul2(tx, P2(da.v, h))), r2);
-            const float2 nz_ = mul2(fma2(d3, fma2(P2(amxz, h), neg, P2(axz, h)), mul2(tz, P2(ca.v, h))), r4);
-            pick2(axx, h, nxx, pxx, m);
-            pick2(azz, h, nzz, pzz, m);
-            sel2(amxz, h, nx_, m.split);
-            pick2(axz, h, add2(nx_, nz_), pxz, m);
+    for (int h = 0; h < NP; h++) {
+        const S2 old{P2(axx, h), P2(azz, h), P2(axz, h)};
+        const S2 pl = as_plain2(old, tx, tz, P2(aa.v, h), P2(ba.v, h), P2(ca.v, h), P2(da.v, h));
+        if (!frame) {
+            W2(axx, h, pl.xx);
+            W2(azz, h, pl.zz);
+            W2(axz, h, pl.xz);
+        } else {
+            // tile with PML cells: the split update in damped cells, the
+            // plain one in the others
+            float2 xp = P2(amxz, h);
+            const S2 sp = as_split2(old, xp, dm.p[h], tx, tz, P2(aa.v, h), P2(ba.v, h), P2(ca.v, h), P2(da.v, h));
+            pick2(axx, h, sp.xx, pl.xx, m);
+            pick2(azz, h, sp.zz, pl.zz, m);
+            sel2(amxz, h, xp, m.split);
+            pick2(axz, h, sp.xz, pl.xz, m);
         }
     }
     stc(p.ad.txx + m.gi, axx);
@@ -1121,19 +960,16 @@ __device__ __forceinline__ void image_lam_mu(const Params &p, const CellMap &m, 
                                              const float axz[CPT], float gl[CPT], float gm[CPT]) {
 #pragma unroll
     for (int h = 0; h < NP; h++) {
-        const float2 gxx = mul2(P2(a.v, h), B2(p.idx)), gzz = mul2(P2(b.v, h), B2(p.idz));
-        const float2 gxz = mul2(P2(cc.v, h), B2(p.idz)), gzx = mul2(P2(d.v, h), B2(p.idx));
-        const float2 x2 = P2(axx, h), z2 = P2(azz, h);
-        // the increments are -lg and -mg (negation is exact)
-        const float2 lg = mul2(add2(gxx, gzz), add2(x2, z2));
-        const float2 mg = fma2(B2(2.f), fma2(gxx, x2, mul2(gzz, z2)), mul2(add2(gxz, gzx), P2(axz, h)));
+        const Img2 g = image2(p.idx, p.idz, P2(a.v, h), P2(b.v, h), P2(cc.v, h), P2(d.v, h),
+                              S2{P2(axx, h), P2(azz, h), P2(axz, h)});
+        const float2 lg = g.lg, mg = g.mg;  // the increments are -lg and -mg (negation is exact)
         float2 ngl, ngm;
         if (w == 1.f) {
             ngl = fma2(B2(-1.f), lg, P2(gl, h));
             ngm = fma2(B2(-1.f), mg, P2(gm, h));
         } else {
-            ngl = add2(P2(gl, h), mul2(B2(-w), lg));
-            ngm = add2(P2(gm, h), mul2(B2(-w), mg));
+            ngl = fma2(B2(-w), lg, P2(gl, h));
+            ngm = fma2(B2(-w), mg, P2(gm, h));
         }
         if (m.image[2 * h]) {
             gl[2 * h] = ngl.x;
@@ -1341,9 +1177,9 @@ __global__ void __launch_bounds__(BLOCK_THREADS, CTAS_PER_SM)
         Damp dm{};
         if (frame) dm = make_damp(p, ex, ez);
         if (frame)
-            s_apply<true>(p, m, p.bg, st, lam, mu, dm, -1.f, a, b, cc, d, nullptr);
+            s_apply<true, false>(p, m, p.bg, st, lam, mu, dm, -1.f, a, b, cc, d, nullptr);
         else
-            s_apply<false>(p, m, p.bg, st, lam, mu, dm, -1.f, a, b, cc, d, nullptr);
+            s_apply<false, false>(p, m, p.bg, st, lam, mu, dm, -1.f, a, b, cc, d, nullptr);
         adjoint_stress(p, m, frame, dm, adj_dir, aa, ba, ca, da, axx, azz, axz, amxz);
         // zero-lag imaging of the lambda and mu kernels (interior cells)
         if (image) {
@@ -1367,11 +1203,13 @@ __device__ __forceinline__ void lame_weight(float *s_P, float *s_Q, float *s_R, 
         f4_to(ld4(s_l + 4 * i), l);
         f4_to(ld4(s_u + 4 * i), u);
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const float l2m = fmaf(2.f, u[j], l[j]);
-            P_[j] = fmaf(l2m, xx[j], l[j] * zz[j]);
-            Q_[j] = fmaf(l[j], xx[j], l2m * zz[j]);
-            R_[j] = u[j] * xz[j];
+        for (int h = 0; h < 2; h++) {
+            const S2 w = lame2(S2{make_float2(xx[2 * h], xx[2 * h + 1]), make_float2(zz[2 * h], zz[2 * h + 1]),
+                                  make_float2(xz[2 * h], xz[2 * h + 1])},
+                               make_float2(l[2 * h], l[2 * h + 1]), make_float2(u[2 * h], u[2 * h + 1]));
+            P_[2 * h] = w.xx.x, P_[2 * h + 1] = w.xx.y;
+            Q_[2 * h] = w.zz.x, Q_[2 * h + 1] = w.zz.y;
+            R_[2 * h] = w.xz.x, R_[2 * h + 1] = w.xz.y;
         }
         st4(s_P + 4 * i, to_f4(P_));
         st4(s_Q + 4 * i, to_f4(Q_));

@@ -37,6 +37,72 @@ const TileVariant *tile_variant_8x32x3();
 const TileVariant *tile_variant_16x32c2();
 const TileVariant *tile_variant_8x32c2s3();
 
+// sfwi_march.cu: whole time steps in one launch.  An item is a strip of
+// zw columns from z0 and the rows [x0, x1) of one shot, one CTA each.
+enum MarchFlags : int {
+    MARCH_SOURCE = 1,  // the source cell lies within 8 cells of the item
+    MARCH_RECV = 2,    // receivers lie in the columns within 8 of the item
+};
+struct alignas(16) MarchItem {
+    int shot, x0, x1, z0, zw, flags;
+    ShotGeo g;
+    int pad[3];
+};
+static_assert(sizeof(MarchItem) == 80, "MarchItem is five 16-byte words");
+// Fields advance from one copy to the other; two fields that advance together
+// (background and scattered; reconstruction and adjoint, both as `bg`) are
+// float2 per cell, a single one (stage 1's forward as `bg`, the adjoint alone as
+// `ad`) is float per cell.
+struct MarchArgs {
+    Params p;  // bg, ad: the copy of the fields that the step writes
+    FieldSet in_bg, in_ad;  // the copy that it reads
+    const MarchItem *items;
+    const float *rsrc;  // residual source [X][rsp]
+    int rsp;
+    const float *fx, *fz;  // PML factors per cell: (d1, r2), (d3, r4)
+    float one;             // 1, not known to the compiler: a product with it must round as any other
+};
+// TMA descriptors of a step, boxes of four rows: the fields read through
+// stencils of the first half-step (view: PS columns), the cells the first
+// half-step updates (rim: PS - 8) and the item's own (core: PS - 16); the digit
+// is the number of consecutive arrays, c: the coefficients (the other maps
+// point at the copy that the step reads, numbered from its first field)
+struct MarchMaps {
+    CUtensorMap view3, view2, rim3, rim2, core2, rim2c, rim1c, core2c, core1c;
+};
+// the fields between the passes: the last forward state becomes the reconstruction
+struct PairStart {
+    const float *src[2];  // the forward steps' copies
+    float *dst[2];        // the backward steps'
+    bool from_pairs, to_pairs;  // (both: in place)
+    int P;
+    size_t cells;
+    const ShotGeo *geo;
+    const ShotAux *aux;
+};
+constexpr int G_ROWS = 4, BURST_ROWS = 16;  // rows of a group; of a burst item at most
+struct MarchVariant {
+    int ps;           // columns of the view; an item has at most ps - 16
+    bool burst;       // an item has at most 16 rows
+    int fwd_ctas[2];  // CTAs per SM: forward (stage 1, Born)
+    int bwd_ctas[2];  // backward (adjoint alone, with the reconstruction)
+    cudaError_t (*configure)();
+    void (*fwd)(const MarchArgs &a, const MarchMaps &tm, int nitems, int it, bool born, cudaStream_t st);
+    void (*bwd)(const MarchArgs &a, const MarchMaps &tm, int nitems, int it, float adj_dir, cudaStream_t st);
+};
+const MarchVariant *march_wide();
+const MarchVariant *march_burst();
+struct MarchFactors {
+    const float *dampx, *dampz;
+    float dt;
+    size_t n;
+    float *fx, *fz;  // float2 per cell
+};
+void launch_march_factors(const MarchFactors &f, cudaStream_t st);
+void launch_pair_start(const PairStart &s, int max_nxpml, int nshots, cudaStream_t st);
+void launch_snap_store(const MarchArgs &a, int max_nxpml, int it, bool pairs, cudaStream_t st);
+void launch_snap_image(const MarchArgs &a, int max_nx, int max_nz, int it, cudaStream_t st);
+
 // sfwi_aux.cu
 struct SetupArgs {
     int X, P, nzpml, pml, allnz, stage, born_lo;

@@ -81,7 +81,9 @@ def strip_steps(nt, strip_chunk=0):
 def request_bytes(req, strip_chunk=0):
     """Device memory of one request's engine (the engine's allocations,
     sfwi_engine.cu:upload_batch, plus the model and the FP64 gradients);
-    strip_chunk > 0: edge strips in host memory in chunks of that many steps."""
+    strip_chunk > 0: edge strips in host memory in chunks of that many steps.
+    The engine's optional second copy of the wavefields is not counted: it is
+    taken only from memory that is plentiful."""
     P = (req.allnz + 2 * req.pml + 3) // 4 * 4
     X = sum(int(d["nx"]) + 2 * req.pml for d in req.shots)
     ntr = sum(len(d["gc"]) for d in req.shots)
