@@ -2012,7 +2012,7 @@ int ot_host(int kind, const float *obs_x, const float *obs_z, const float *cal_x
         o.sigma = dd;
         o.trace_misfit = dd + 2 * tracenum;
         o.scratch = nscr ? dd + 4 * (size_t)tracenum : nullptr;
-        if ((e = launch_ot(o, 0)) != cudaSuccess) break;
+        if ((e = launch_ot_gather(o, 0)) != cudaSuccess) break;
         if ((e = cudaMemcpy(res_z, d + 4 * n, n * 4, cudaMemcpyDeviceToHost)) != cudaSuccess) break;
         if ((e = cudaMemcpy(res_x, d + 5 * n, n * 4, cudaMemcpyDeviceToHost)) != cudaSuccess) break;
         if ((e = cudaMemcpy(tm.data(), dd + 2 * tracenum, tm.size() * 8, cudaMemcpyDeviceToHost)) != cudaSuccess) break;

@@ -157,8 +157,9 @@ struct OtArgs {
     double *trace_misfit;         // [ntr][2]
     double *scratch;              // traces longer than ot_max_nt(): ot_scratch_doubles(nt, ntr) doubles
 };
+// the adjoint source of a gradient run; a gather's misfit by itself (sfwi_ot, sfwi_ot_noalloc)
 cudaError_t launch_ot(const OtArgs &a, cudaStream_t st);
-size_t ot_smem_bytes(int nt);
+cudaError_t launch_ot_gather(const OtArgs &a, cudaStream_t st);
 // longest trace held in shared memory; longer ones need the global scratch
 int ot_max_nt();
 size_t ot_scratch_doubles(int nt, int ntr);

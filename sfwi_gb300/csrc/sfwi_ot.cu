@@ -15,14 +15,31 @@
 //   adjoint   A_j = ((j+1)dt - T_j)^2 - 2 sum_{k>=j} ((k+1)dt - T_k) f_k dt / g_m(k)
 //             res_i = (1/2) (A_i - sum_j f_j A_j) / sum p(cal) * p'(cal_i)
 // res is (1/2) dW/dcal, the scaling of the L2 residual (misfit sum r^2,
-// adjoint source r).  The CDFs, the quantile search and every sum are FP64.
-// The exponential weights are FP32 (expf of the argument rounded to FP32,
-// then widened): their argument is at most 0, so a weight is 1 at the
-// trace's maximum and its relative rounding of about 1e-7 stays far below
-// the 1e-4 parity bar, while a double exp would be most of the kernel's
-// FP64 work.
+// adjoint source r).
+//
+// Two kernels.  k_ot_fp64 forms the adjoint sources of gradient runs, all sums,
+// products and divisions in FP64 (the FP64 pipe, 1/64 of the FP32 rate, is 86 % busy:
+// 2.87 ms for both components of 3760 traces of 3000 samples; 1 to 2 % of a gradient run).
+// k_ot serves the calls that want a gather's misfit and residuals by themselves
+// and takes 0.47 ms: there the CDFs are 64-bit integers and the rest is in float
+// pairs.  Its residuals differ from k_ot_fp64's in the last bit of one in 2000, which is
+// nothing by itself; but an FP32 propagation of that source ends 7e-6 away from
+// the other's after 3000 steps (as far as each is from FP64), so gradient
+// runs stay with the FP64 form and their bits.
+// The integers: CDFs are sums of positive weights, in units of 2^-s of the
+// largest one, s such that a trace's sum stays below 2^62.  Integer sums are
+// exact in any order, so F_k - G_{m-1} and the search have no rounding but the weights'
+// own (2^-50 at 3000 samples), and equal traces have equal CDFs.  What
+// follows the search (r, its square, the adjoint weights and their sums) is in
+// float pairs of 48 bits (see D2); its cancellation of nearly equal numbers,
+// k+1 - T_k, is done in integers before.  Against FP64 the errors are those of the FP64
+// kernel: residuals the same to six digits, misfits at 1e-14.
+// In both the exponential weights are FP32 (expf of the argument rounded to FP32):
+// their argument is at most 0, so a weight is 1 at the trace's maximum and
+// its relative rounding of about 1e-7 stays far below the 1e-4 parity bar.
 // One CTA handles one (trace, component); prefix and suffix sums are block
 // scans built on warp shuffles.
+#include <algorithm>
 #include <cfloat>
 #include <cudaTypedefs.h>
 #include <mutex>
@@ -31,7 +48,9 @@
 
 namespace sfwi {
 
-constexpr int OT_THREADS = 256;
+using u64 = unsigned long long;
+
+constexpr int OT_THREADS = 256;  // of k_ot_fp64
 
 __device__ __forceinline__ double warp_incl_scan(double v) {
     const int l = threadIdx.x & 31;
@@ -72,33 +91,6 @@ __device__ double block_reduce(double v, double *wsum) {
     return t;
 }
 
-__device__ double block_max(double v, double *wsum) {
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (l == 0) wsum[w] = v;
-    __syncthreads();
-    double t = -DBL_MAX;
-    for (int i = 0; i < (int)(blockDim.x >> 5); i++) t = fmax(t, wsum[i]);
-    __syncthreads();
-    return t;
-}
-
-// in-place inclusive prefix (reverse=false) or suffix (reverse=true) sums of a[0..n)
-__device__ void block_scan_array(double *a, int n, bool reverse, double *wsum) {
-    const int chunk = (n + blockDim.x - 1) / blockDim.x;
-    const int b = threadIdx.x * chunk, e = min(n, b + chunk);
-    double s = 0.0;
-    for (int i = b; i < e; i++) s += a[reverse ? n - 1 - i : i];
-    const double off = block_excl_scan(s, wsum);
-    double run = off;
-    for (int i = b; i < e; i++) {
-        const int k = reverse ? n - 1 - i : i;
-        run += a[k];
-        a[k] = run;
-    }
-    __syncthreads();
-}
-
 // exclusive suffix sums over the threads of the block: thread t gets the sum
 // of v over threads t+1 .. blockDim.x-1 (cs: blockDim.x doubles of shared
 // memory; wsum as block_excl_scan)
@@ -114,11 +106,161 @@ __device__ double block_excl_suffix(double v, double *cs, double *wsum) {
     return r;
 }
 
+// ---------------------------------------------------------------------------
+// float pairs: the unevaluated sum h + l of two floats, |l| <= ulp(h)/2
+// (Dekker 1971, Knuth's two-sum; the product's error term by FMA)
+// ---------------------------------------------------------------------------
+struct D2 {
+    float h, l;
+};
+__device__ __forceinline__ D2 quick2(float a, float b) {  // |a| >= |b| or a = 0
+    const float s = __fadd_rn(a, b);
+    return D2{s, __fadd_rn(b, -__fadd_rn(s, -a))};
+}
+__device__ __forceinline__ D2 sum2(float a, float b) {
+    const float s = __fadd_rn(a, b), t = __fadd_rn(s, -a);
+    return D2{s, __fadd_rn(__fadd_rn(a, -__fadd_rn(s, -t)), __fadd_rn(b, -t))};
+}
+__device__ __forceinline__ D2 operator+(D2 a, D2 b) {  // to 2^-47 (|a| + |b|)
+    const D2 s = sum2(a.h, b.h);
+    return quick2(s.h, __fadd_rn(s.l, __fadd_rn(a.l, b.l)));
+}
+__device__ __forceinline__ D2 operator-(D2 a) { return D2{-a.h, -a.l}; }
+__device__ __forceinline__ D2 operator*(D2 a, D2 b) {
+    const float p = __fmul_rn(a.h, b.h);
+    float e = __fmaf_rn(a.h, b.h, -p);
+    e = __fmaf_rn(a.h, b.l, e);
+    e = __fmaf_rn(a.l, b.h, e);
+    return quick2(p, e);
+}
+__device__ __forceinline__ D2 reciprocal(D2 d) {
+    // two terms of the series from an approximate reciprocal of the high part
+    const float x = __fdividef(1.f, d.h);
+    float e = __fmaf_rn(-d.h, x, 1.f);
+    e = __fmaf_rn(-d.l, x, e);
+    return quick2(x, __fmul_rn(x, __fmaf_rn(e, e, e)));
+}
+__device__ __forceinline__ D2 to_d2(double v) {
+    const float h = (float)v;
+    return D2{h, (float)(v - (double)h)};
+}
+__device__ __forceinline__ double to_f64(D2 a) { return (double)a.h + (double)a.l; }
+// an integer below 2^63, to 48 bits
+__device__ __forceinline__ D2 to_d2(u64 x) {
+    const float a = (float)(unsigned)(x >> 40), b = (float)((unsigned)(x >> 16) & 0xffffffu),
+                c = (float)((unsigned)x & 0xffffu);
+    const D2 s = quick2(a * 1099511627776.f, b * 65536.f);
+    return quick2(s.h, __fadd_rn(s.l, c));
+}
+__device__ __forceinline__ D2 to_d2(long long x) {
+    const D2 m = to_d2((u64)(x < 0 ? -x : x));
+    return x < 0 ? -m : m;
+}
+// x 2^s of a float 0 <= x <= 1 (24 <= s <= 62), rounded
+__device__ __forceinline__ u64 fixed_point(float x, int s) {
+    const unsigned b = __float_as_uint(x), e = b >> 23;
+    const u64 m = (u64)((b & 0x7fffffu) | 0x800000u) << (s - 22);
+    return e == 0 ? 0 : ((m >> min(127u - e, 63u)) + 1) >> 1;
+}
+
+// ---------------------------------------------------------------------------
+// block sums (blockDim.x a multiple of 32); `sm`: 66 64-bit words, not read
+// by other threads when a call begins
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ D2 shfl_down(D2 v, int o) {
+    return D2{__shfl_down_sync(0xffffffffu, v.h, o), __shfl_down_sync(0xffffffffu, v.l, o)};
+}
+// exclusive sums over the threads before this one, of two values at once; the
+// totals go to sm[64], sm[65] (the second level of these sums is one warp's work: done by
+// every thread it was a quarter of the kernel's instructions)
+__device__ void block_scan2(u64 &a, u64 &b, u64 *sm) {
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+    auto warp_scan = [&](u64 &x, u64 &y) {
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const u64 u = __shfl_up_sync(0xffffffffu, x, o), v = __shfl_up_sync(0xffffffffu, y, o);
+            if (l >= o) x += u, y += v;
+        }
+    };
+    u64 x = a, y = b;
+    warp_scan(x, y);
+    if (l == 31) sm[w] = x, sm[32 + w] = y;
+    __syncthreads();
+    if (w == 0) {
+        const u64 p = l < nw ? sm[l] : 0, q = l < nw ? sm[32 + l] : 0;
+        u64 u = p, v = q;
+        warp_scan(u, v);
+        sm[l] = u - p, sm[32 + l] = v - q;
+        if (l == 31) sm[64] = u, sm[65] = v;
+    }
+    __syncthreads();
+    a = sm[w] + x - a;
+    b = sm[32 + w] + y - b;
+}
+// the sum over the threads after this one
+__device__ D2 block_suffix(D2 v, u64 *sm) {
+    D2 *ws = reinterpret_cast<D2 *>(sm);
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+    auto warp_suffix = [&](D2 x) {  // this lane's and those after it
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const D2 u = shfl_down(x, o);
+            if (l + o < 32) x = x + u;
+        }
+        return x;
+    };
+    auto drop_own = [&](D2 x) {
+        x = shfl_down(x, 1);
+        return l == 31 ? D2{0.f, 0.f} : x;
+    };
+    const D2 x = warp_suffix(v), after = drop_own(x);
+    if (l == 0) ws[w] = x;
+    __syncthreads();
+    if (w == 0) {
+        const D2 t = drop_own(warp_suffix(l < nw ? ws[l] : D2{0.f, 0.f}));
+        ws[l] = t;
+    }
+    __syncthreads();
+    return after + ws[w];
+}
+// the sums of two values; valid in thread 0
+__device__ void block_sum2(D2 &v, D2 &u, u64 *sm) {
+    D2 *ws = reinterpret_cast<D2 *>(sm);
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+    auto warp_sum = [&](D2 x) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x = x + shfl_down(x, o);
+        return x;
+    };
+    v = warp_sum(v), u = warp_sum(u);
+    if (l == 0) ws[w] = v, ws[32 + w] = u;
+    __syncthreads();
+    if (w == 0) {
+        v = warp_sum(l < nw ? ws[l] : D2{0.f, 0.f});
+        u = warp_sum(l < nw ? ws[32 + l] : D2{0.f, 0.f});
+    }
+}
+__device__ __forceinline__ float warp_max(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_down_sync(0xffffffffu, v, o));
+    return v;
+}
+__device__ double block_max(double v, double *wsum) {
+    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    if (l == 0) wsum[w] = v;
+    __syncthreads();
+    double t = -DBL_MAX;
+    for (int i = 0; i < (int)(blockDim.x >> 5); i++) t = fmax(t, wsum[i]);
+    __syncthreads();
+    return t;
+}
+
 // smallest m >= lo with G[m] > y, capped at n-1 (G non-decreasing and every
 // index below lo known to hold G <= y): a galloping search from lo, so
 // consecutive quantiles of one thread cost a few probes instead of a full
 // binary search; the answer is that of a binary search over [0, n-1)
-__device__ __forceinline__ int first_above(const double *G, int n, double y, int lo) {
+__device__ __forceinline__ int first_above(const u64 *G, int n, u64 y, int lo) {
     if (lo >= n - 1) return n - 1;
     if (G[lo] > y) return lo;
     int prev = lo, step = 1, hi;
@@ -146,6 +288,9 @@ __device__ __forceinline__ int first_above(const double *G, int n, double y, int
     return l;
 }
 
+// ---------------------------------------------------------------------------
+// the FP64 form, for gradient runs
+// ---------------------------------------------------------------------------
 // The GB300's FP64 rate is a small fraction of its FP32 rate, so the kernel
 // spends FP64 operations sparingly: each thread owns one contiguous chunk of
 // samples, the positivity transform (one exp per sample and trace) is
@@ -160,7 +305,7 @@ constexpr int OT_MAX_CHUNK = 32;  // samples per thread of the shared-memory for
 // arrays of nt doubles per (trace, component), for longer traces (the
 // transport residuals r then go to the fifth array instead of registers).
 template <bool LONG>
-__global__ void __launch_bounds__(OT_THREADS) k_ot(OtArgs a) {
+__global__ void __launch_bounds__(OT_THREADS) k_ot_fp64(OtArgs a) {
     extern __shared__ double ot_sm[];
     __shared__ double wsum[32];
     __shared__ double cs[OT_THREADS];
@@ -184,10 +329,10 @@ __global__ void __launch_bounds__(OT_THREADS) k_ot(OtArgs a) {
     const int chunk = (n + blockDim.x - 1) / blockDim.x;
     const int k0 = min(n, (int)threadIdx.x * chunk), k1 = min(n, k0 + chunk);
 
-    double mc = -DBL_MAX, mo = -DBL_MAX;
+    float mc = -FLT_MAX, mo = -FLT_MAX;
     for (int k = k0; k < k1; k++) {
-        mc = fmax(mc, pred(k));
-        mo = fmax(mo, (double)obs[k]);
+        mc = fmaxf(mc, cal2 ? cal[k] + cal2[k] : cal[k]);
+        mo = fmaxf(mo, obs[k]);
     }
     const double cmax = block_max(mc, wsum), omax = block_max(mo, wsum);
     const double eps = 1e-3 * sigma * sigma;
@@ -229,7 +374,7 @@ __global__ void __launch_bounds__(OT_THREADS) k_ot(OtArgs a) {
         const int k = k0 + i;
         const double fk = P[k] * inv_Sf;
         Fk += fk;
-        m = first_above(G, n, Fk, m);
+        m = first_above(reinterpret_cast<const u64 *>(G), n, (u64)__double_as_longlong(Fk), m);  // (order of the bits)
         const double gm = g[m];
         const double inv_gm = 1.0 / gm;
         const double Gm1 = m > 0 ? G[m - 1] : 0.0;
@@ -265,10 +410,227 @@ __global__ void __launch_bounds__(OT_THREADS) k_ot(OtArgs a) {
     if (threadIdx.x == 0) a.trace_misfit[2 * tr + comp] = W;
 }
 
-size_t ot_smem_bytes(int nt) { return (size_t)4 * nt * sizeof(double); }
+// ---------------------------------------------------------------------------
+// integers and float pairs, for a gather's misfit by itself
+// ---------------------------------------------------------------------------
+// LONG = false: the per-trace arrays in shared memory (traces up to
+// ot_max_nt() samples); LONG = true: in the caller's global scratch, five
+// arrays of nt doubles per (trace, component), for longer traces.
+// POWER: OT_power's weights, in units of sigma^2: v^2 + 1e-3 with v = u / sigma.
+// Each thread owns one contiguous run of an odd number of samples (`run`), so that the
+// threads' accesses to 64-bit arrays in shared memory fall into different
+// banks; the quantile search continues from the previous sample's.
+// Bound by instructions (470 us for 3760 traces of 3000 samples, 64 % of the issue slots, DRAM 7 %); 56
+// registers let three CTAs of 352 threads share an SM (64: two, 685 us for 590).
+template <bool LONG, bool POWER>
+__global__ void __maxnreg__(56) k_ot(OtArgs a, int run) {
+    extern __shared__ u64 ot_words[];
+    // block sums; a call's words may be read until the next barrier, so calls alternate
+    __shared__ u64 ws[2][66];
+    // per-trace constants, formed by thread 0 in FP64
+    __shared__ struct {
+        float mc, mo;
+        double inv_sigma, scale;
+        D2 is, c, norm, sc, FA;
+        u64 ratio;
+        int wide, ec, eo, bc, bo, shift;
+    } tc;
+    const int n = a.nt;
+    // G: CDF of the observed trace; B: the adjoint weights but for a constant
+    // per thread (first: obs); U: p(cal), POWER: cal
+    u64 *G = LONG ? reinterpret_cast<u64 *>(a.scratch) + (size_t)blockIdx.x * 5 * n : ot_words;
+    D2 *B = reinterpret_cast<D2 *>(G + n);
+    float *U = reinterpret_cast<float *>(B + n), *O = reinterpret_cast<float *>(B);
+    const int tr = blockIdx.x >> 1, comp = blockIdx.x & 1;
+    const size_t o = (size_t)tr * n;
+    const float *cal = (comp ? a.cal_x : a.cal_z) + o;
+    const float *cal2 = a.cal2_z ? (comp ? a.cal2_x : a.cal2_z) + o : nullptr;
+    const float *obs = (comp ? a.obs_x : a.obs_z) + o;
+    float *res = (comp ? a.res_x : a.res_z) + o;
+    // both traces (obs in B's place until its weights are taken), their
+    // largest values and magnitudes
+    float mc = -FLT_MAX, mo = -FLT_MAX, ac = 0.f, ao = 0.f;
+#pragma unroll 4
+    for (int k = threadIdx.x; k < n; k += blockDim.x) {
+        const float u = cal2 ? cal[k] + cal2[k] : cal[k], v = obs[k];
+        U[k] = u;
+        O[k] = v;
+        mc = fmaxf(mc, u), ac = fmaxf(ac, fabsf(u));
+        mo = fmaxf(mo, v), ao = fmaxf(ao, fabsf(v));
+    }
+    // units of the weights: 2^-bits of 2^ec, 2^eo, the powers of two above them
+    const int all_ones = 62 - (32 - __clz((n - 1) | 1));
+    int bc = all_ones, bo = all_ones;
+    {
+        float *w = reinterpret_cast<float *>(ws[0]);
+        mc = warp_max(mc), mo = warp_max(mo), ac = warp_max(ac), ao = warp_max(ao);
+        const int l = threadIdx.x & 31, nw = blockDim.x >> 5;
+        if (l == 0) {
+            float *q = w + 4 * (threadIdx.x >> 5);
+            q[0] = mc, q[1] = mo, q[2] = ac, q[3] = ao;
+        }
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            mc = warp_max(l < nw ? w[4 * l] : -FLT_MAX), mo = warp_max(l < nw ? w[4 * l + 1] : -FLT_MAX);
+            ac = warp_max(l < nw ? w[4 * l + 2] : 0.f), ao = warp_max(l < nw ? w[4 * l + 3] : 0.f);
+        }
+    }
+    if (threadIdx.x == 0) {
+        double sigma = a.sigma[2 * tr + comp];
+        if (!(sigma > 0.0)) sigma = 1.0;
+        const double inv = 1.0 / sigma;
+        tc.mc = mc, tc.mo = mo;
+        tc.inv_sigma = inv;
+        tc.is = to_d2(inv);
+        // Scales at which a float pair could overflow or lose bits: the
+        // weights' arguments and the last product are then formed in FP64.
+        tc.wide = !(sigma > 1e-15 && sigma < 1e15 && fmaxf(ac, ao) < 1e9 * sigma);
+        tc.ec = tc.eo = 0;
+        if (POWER) {
+            // (no finite magnitude: every weight is NaN, and the result)
+            frexp(ac * inv * (ac * inv) + 1e-3, &tc.ec);
+            frexp(ao * inv * (ao * inv) + 1e-3, &tc.eo);
+        }
+    }
+    __syncthreads();
+    mc = tc.mc, mo = tc.mo;
+    const int ec = tc.ec, eo = tc.eo;
+    const bool wide = tc.wide;
+    const double inv_sigma = tc.inv_sigma;
+    const D2 is = tc.is;
+    if (POWER && !wide) {
+        // A few large samples and many near 1e-3: the sum of the weights is
+        // far below their number, which leaves bits for the small ones.
+        const float qc = __int_as_float((127 - ec) << 23), qo = __int_as_float((127 - eo) << 23);
+        float x = 0.f, y = 0.f;
+        for (int k = threadIdx.x; k < n; k += blockDim.x) {
+            const float u = U[k] * is.h, v = O[k] * is.h;
+            x += (u * u + 1e-3f) * qc, y += (v * v + 1e-3f) * qo;
+        }
+        D2 sx{x, 0.f}, sy{y, 0.f};
+        block_sum2(sx, sy, ws[1]);
+        if (threadIdx.x == 0) {
+            // (a margin for the rounding of these sums)
+            auto room = [&](float t) { return t > 0.f ? min(max(all_ones, 62 - (ilogbf(1.01f * t) + 1)), 62) : all_ones; };
+            tc.bc = room(sx.h), tc.bo = room(sy.h);
+        }
+        __syncthreads();
+        bc = tc.bc, bo = tc.bo;
+    }
+    auto weight = [&](float u, float top, int e) -> D2 {
+        if (POWER) {
+            if (wide) {
+                const double v = u * inv_sigma;
+                return to_d2(ldexp(v * v + 1e-3, -e));
+            }
+            D2 v = is * D2{u, 0.f};
+            v = v * v + D2{1e-3f, (float)(1e-3 - (double)1e-3f)};
+            const float c = __int_as_float((127 - e) << 23);
+            return D2{v.h * c, v.l * c};
+        }
+        if (wide) return D2{expf((float)(((double)u - (double)top) * inv_sigma)), 0.f};
+        const D2 d = sum2(u, -top) * is;
+        return D2{expf(d.h + d.l), 0.f};
+    };
+    auto units = [&](D2 w, int bits) -> u64 {
+        u64 x = fixed_point(w.h, bits);
+        if (POWER) x = w.l < 0.f ? x - fixed_point(-w.l, bits) : x + fixed_point(w.l, bits);
+        return x;
+    };
+    const int k0 = min(n, (int)threadIdx.x * run), k1 = min(n, k0 + run);
 
-// longest trace k_ot takes: four FP64 arrays of nt samples next to the static
-// block-scan buffers within 227 KB, and at most OT_MAX_CHUNK samples a thread
+    // weights, the sums of both runs, and the CDF G of the observed trace
+    u64 F = 0, offG = 0;
+    bool bad = false;
+    for (int k = k0; k < k1; k++) {
+        const D2 x = weight(U[k], mc, ec), y = weight(O[k], mo, eo);
+        bad |= !(x.h <= 2.f && y.h <= 2.f);
+        if (!POWER) U[k] = x.h;
+        F += units(x, bc);
+        offG += units(y, bo);
+        G[k] = offG;
+    }
+    bad = __syncthreads_or(bad);
+    block_scan2(F, offG, ws[1]);
+    for (int k = k0; k < k1; k++) G[k] += offG;
+    if (threadIdx.x == 0) {
+        const double sf = (double)ws[1][64], sg = (double)ws[1][65], q = sg / sf;
+        // ratio of the units, SG / SF = (ratio / 2^63) 2^shift
+        const u64 rb = (u64)__double_as_longlong(q);
+        tc.ratio = ((rb & 0xfffffffffffffULL) | 0x10000000000000ULL) << 11;
+        tc.shift = (int)(rb >> 52) - 1023;
+        // f / g = (p / SF) (SG / g), p and g in their units
+        tc.c = to_d2(-2.0 * ldexp(q, bc));
+        // sums of weights are SF 2^-bc
+        const double inv_S = ldexp(1.0 / sf, bc);
+        tc.norm = to_d2(-inv_S);
+        // res = (1/2) (A - FA) / S p'(u): p' = p / sigma, or (POWER, p in units
+        // of 2^ec sigma^2) 2 (u / sigma) / sigma
+        tc.scale = a.dt * a.dt * inv_S * (POWER ? ldexp(1.0, -ec) : 0.5);
+        tc.sc = to_d2(tc.scale);
+    }
+    __syncthreads();
+    if (bad) {
+        // a weight without a finite value leaves none in the trace
+        for (int k = threadIdx.x; k < n; k += blockDim.x) res[k] = __int_as_float(0x7fffffff);
+        if (threadIdx.x == 0) a.trace_misfit[2 * tr + comp] = __longlong_as_double(0x7fffffffffffffffLL);
+        return;
+    }
+    auto p_of = [&](int k) -> D2 { return POWER ? weight(U[k], mc, ec) : D2{U[k], 0.f}; };
+
+    // transport, in samples: r_k = k + 1 - T_k = i - (F_k - G_{m-1}) / g_m, i = k + 1 - m
+    // Adjoint weights in samples squared: A_k = r_k^2 + c sum_{j>=k} q_j, q_j = r_j p_j / g_m(j).
+    // The sum is the block's after this thread's samples, plus the thread's own less what
+    // comes before k, so a thread keeps B_k = r_k^2 - c sum_{j<k} q_j and adds a
+    // constant when the block's sums are known.
+    const u64 ratio = tc.ratio, SF = ws[1][64], SG = ws[1][65];
+    const int shift = tc.shift;
+    const D2 c = tc.c;
+    D2 w{0.f, 0.f}, sq{0.f, 0.f}, fb{0.f, 0.f}, sp{0.f, 0.f};
+    int m = 0;
+    for (int k = k0; k < k1; k++) {
+        const D2 pk = p_of(k);
+        F += units(pk, bc);
+        u64 y = __umul64hi(F << 1, ratio);
+        y = shift >= 0 ? y << min(shift, 63) : y >> min(-shift, 63);
+        if (F == SF) y = SG;  // (the ratio is rounded)
+        m = first_above(G, n, y, m);
+        const u64 below = m > 0 ? G[m - 1] : 0, g = G[m] - below;
+        // (r of -1 to 1 from integers alone: near equal traces lose nothing)
+        const int i = k + 1 - m;
+        const u64 num = i == 1 ? g - (y - below) : y - below;
+        const D2 ig = reciprocal(to_d2(g)), q1 = to_d2((long long)(i == 1 ? num : 0 - num)) * ig;
+        const D2 r = i == 0 || i == 1 ? q1 : D2{(float)i, 0.f} + q1, rr = r * r;
+        const D2 b = rr + -(c * sq);
+        B[k] = b;
+        w = w + pk * rr;
+        fb = fb + pk * b;
+        sp = sp + pk;
+        sq = sq + pk * r * ig;
+    }
+    const D2 rest = c * (block_suffix(sq, ws[0]) + sq);
+    fb = fb + rest * sp;
+    block_sum2(fb, w, ws[1]);
+    if (threadIdx.x == 0) {
+        tc.FA = fb * tc.norm;
+        a.trace_misfit[2 * tr + comp] = -to_f64(w * tc.norm) * a.dt * a.dt;
+    }
+    __syncthreads();
+    const D2 FA = tc.FA, sc = tc.sc;
+    for (int k = k0; k < k1; k++) {
+        const D2 d = (B[k] + rest) + FA, x{U[k], 0.f};
+        if (wide) {
+            res[k] = (float)(to_f64(d) * tc.scale * (POWER ? inv_sigma * U[k] : U[k]) * inv_sigma);
+        } else {
+            const D2 v = d * sc * (POWER ? is * x : x) * is;
+            res[k] = v.h + v.l;
+        }
+    }
+}
+
+// longest trace held in shared memory: four FP64 arrays of nt samples next to the
+// static block-scan buffers within 227 KB, and at most OT_MAX_CHUNK samples a
+// thread (k_ot, which needs 20 bytes a sample, keeps the same limit)
 int ot_max_nt() {
     const int by_smem = (int)((227 * 1024 - (OT_THREADS + 32) * sizeof(double) - 1024) / (4 * sizeof(double)));
     return by_smem < OT_MAX_CHUNK * OT_THREADS ? by_smem : OT_MAX_CHUNK * OT_THREADS;
@@ -276,17 +638,48 @@ int ot_max_nt() {
 
 size_t ot_scratch_doubles(int nt, int ntr) { return nt > ot_max_nt() ? (size_t)5 * nt * 2 * ntr : 0; }
 
+template <bool LONG, bool POWER>
+static cudaError_t launch_ot_form(const OtArgs &a, cudaStream_t st) {
+    // Runs of an odd number of samples, at most 512 threads.  3760 traces of 3000 samples
+    // (both components): runs of 7, 9, 11, 13, 15 samples 660, 585, 590, 606, 650 us, each thread's share
+    // of the block sums (about four samples' work) against the threads that hide
+    // latency; 8000 of 300 samples: 5, 7, 9, 11 samples 192, 217, 241, 191 us, by the
+    // warps' idle threads.  Few traces want many threads each (37 of 120 samples: 3
+    // samples 57 us, 9 samples 65 us).
+    const int least = (a.nt + 511) / 512 | 1;
+    auto threads_of = [&](int r) { return ((a.nt + r - 1) / r + 31) & ~31; };
+    int run = std::max(3, least);
+    if (a.ntr >= 256)
+        for (int r = run = std::max(5, least); r <= 11; r += 2)
+            if (threads_of(r) * (r + 4) < threads_of(run) * (run + 4)) run = r;
+    const int threads = threads_of(run);
+    const size_t sm = LONG ? 0 : (size_t)a.nt * 20;
+    if (!LONG) {
+        cudaError_t e = cudaFuncSetAttribute(k_ot<LONG, POWER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        if (e != cudaSuccess) return e;
+    }
+    k_ot<LONG, POWER><<<2 * a.ntr, threads, sm, st>>>(a, run);
+    return cudaGetLastError();
+}
 cudaError_t launch_ot(const OtArgs &a, cudaStream_t st) {
     if (a.nt > ot_max_nt()) {
         if (!a.scratch) return cudaErrorInvalidValue;
-        k_ot<true><<<2 * a.ntr, OT_THREADS, 0, st>>>(a);
+        k_ot_fp64<true><<<2 * a.ntr, OT_THREADS, 0, st>>>(a);
         return cudaGetLastError();
     }
-    const size_t sm = ot_smem_bytes(a.nt);
-    cudaError_t e = cudaFuncSetAttribute(k_ot<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    const size_t sm = (size_t)4 * a.nt * sizeof(double);
+    cudaError_t e = cudaFuncSetAttribute(k_ot_fp64<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
-    k_ot<false><<<2 * a.ntr, OT_THREADS, sm, st>>>(a);
+    k_ot_fp64<false><<<2 * a.ntr, OT_THREADS, sm, st>>>(a);
     return cudaGetLastError();
+}
+cudaError_t launch_ot_gather(const OtArgs &a, cudaStream_t st) {
+    const bool power = a.kind == 2;
+    if (a.nt > ot_max_nt()) {
+        if (!a.scratch) return cudaErrorInvalidValue;
+        return power ? launch_ot_form<true, true>(a, st) : launch_ot_form<true, false>(a, st);
+    }
+    return power ? launch_ot_form<false, true>(a, st) : launch_ot_form<false, false>(a, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -307,15 +700,23 @@ constexpr int OT_NOALLOC_MAX_TRACES = 8192;
 // (trace, component); [4*max]: the summed misfit
 static __device__ __align__(256) double g_ot_noalloc_scratch[4 * OT_NOALLOC_MAX_TRACES + 32];
 
-// scale of trace `blockIdx.x>>1`, component `blockIdx.x&1`: max |obs|
+// scale of trace `blockIdx.x>>1`, component `blockIdx.x&1`: max |obs| (a
+// maximum of floats is exact: FP64 comparisons took 137 us for 3760 traces of 3000
+// samples, now 44 us)
 __global__ void k_ot_trace_scale(const float *obs_z, const float *obs_x, int nt, double *sigma) {
-    __shared__ double wsum[32];
+    __shared__ float wm[32];
     const int tr = blockIdx.x >> 1, comp = blockIdx.x & 1;
     const float *o = (comp ? obs_x : obs_z) + (size_t)tr * nt;
-    double m = 0.0;
-    for (int k = threadIdx.x; k < nt; k += blockDim.x) m = fmax(m, fabs((double)o[k]));
-    const double t = block_max(m, wsum);
-    if (threadIdx.x == 0) sigma[blockIdx.x] = t;
+    float m = 0.f;
+#pragma unroll 4
+    for (int k = threadIdx.x; k < nt; k += blockDim.x) m = fmaxf(m, fabsf(o[k]));
+    m = warp_max(m);
+    if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < (int)(blockDim.x >> 5); i++) m = fmaxf(m, wm[i]);
+        sigma[blockIdx.x] = m;
+    }
 }
 
 // gather-wide scale: every trace of a component takes the largest (kind 3),
@@ -354,13 +755,19 @@ void launch_ot_scales(const float *obs_z, const float *obs_x, int nt, int ntr, c
     k_ot_shot_scale<<<2 * nshots, 256, 0, st>>>(sigma, geo, all);
 }
 
-// misfit = sum over traces of the two components, in trace order
-__global__ void k_ot_sum(const double *trace_misfit, int ntr, double *out) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double w = 0.0;
-        for (int i = 0; i < 2 * ntr; i++) w += trace_misfit[i];
-        *out = w;
+// misfit = sum over traces of the two components: 1024 partial sums in trace order,
+// then a fixed tree (one thread's chain of 7520 additions took 450 us, this 10 us)
+__global__ void __launch_bounds__(1024) k_ot_sum(const double *trace_misfit, int ntr, double *out) {
+    __shared__ double p[1024];
+    double w = 0.0;
+    for (int i = threadIdx.x; i < 2 * ntr; i += 1024) w += trace_misfit[i];
+    p[threadIdx.x] = w;
+    __syncthreads();
+    for (int h = 512; h > 0; h >>= 1) {
+        if (threadIdx.x < h) p[threadIdx.x] += p[threadIdx.x + h];
+        __syncthreads();
     }
+    if (threadIdx.x == 0) *out = p[0];
 }
 
 }  // namespace sfwi
@@ -459,8 +866,8 @@ extern "C" int sfwi_ot_noalloc(int kind, const float *obs_x, const float *obs_z,
     o.res_x = res_x;
     o.sigma = sigma;
     o.trace_misfit = tmis;
-    if ((e = launch_ot(o, st)) != cudaSuccess) return record_error(-2, "sfwi_ot_noalloc: %s", cudaGetErrorString(e));
-    k_ot_sum<<<1, 32, 0, st>>>(tmis, tracenum, sum);
+    if ((e = launch_ot_gather(o, st)) != cudaSuccess) return record_error(-2, "sfwi_ot_noalloc: %s", cudaGetErrorString(e));
+    k_ot_sum<<<1, 1024, 0, st>>>(tmis, tracenum, sum);
     double w = 0.0;
     if ((e = cudaMemcpyAsync(&w, sum, sizeof(double), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
         (e = cudaStreamSynchronize(st)) != cudaSuccess)
