@@ -332,7 +332,8 @@ struct sfwi_handle {
     // exact Born adjoint (sfwi_born_adjoint): adjoint state and gathered
     // fields, accumulators, per-row shot and receiver tables, the image
     DevBuf<float> adj_f;
-    DevBuf<double> adj_d, adj_img;
+    DevBuf<float2> adj_d;
+    DevBuf<double> adj_img;
     DevBuf<int> adj_i;
 };
 
@@ -1844,10 +1845,10 @@ int born_adjoint(sfwi_handle *h, const std::vector<ShotIn> &q, double *img_vp, d
     // adjoint workspace: 18 float fields, 2 double accumulators, tables
     const size_t cells = b.cells, gcells = (size_t)h->allnx * h->allnz;
     CK(h->adj_f.ensure(18 * cells));
-    CK(h->adj_d.ensure(2 * cells));
+    CK(h->adj_d.ensure(2 * cells + 1));  // and the peaks
     CK(h->adj_img.ensure(2 * gcells));
     CK(cudaMemsetAsync(h->adj_f.p, 0, 18 * cells * sizeof(float), st));
-    CK(cudaMemsetAsync(h->adj_d.p, 0, 2 * cells * sizeof(double), st));
+    CK(cudaMemsetAsync(h->adj_d.p, 0, (2 * cells + 1) * sizeof(float2), st));
     CK(cudaMemsetAsync(h->adj_img.p, 0, 2 * gcells * sizeof(double), st));
     // per packed row: its shot, and the traces recorded at its receiver cell
     std::vector<int> tab(b.X + (b.X + 1) + std::max(b.ntr_tot, 1), 0);
@@ -1869,7 +1870,6 @@ int born_adjoint(sfwi_handle *h, const std::vector<ShotIn> &q, double *img_vp, d
     a.PS = b.PS;
     a.pml = h->pml;
     a.nt = nt;
-    a.born_lo = NOP;
     a.dt = h->dt;
     a.dtdx = h->dt / h->dx;
     a.dtdz = h->dt / h->dz;
@@ -1890,13 +1890,13 @@ int born_adjoint(sfwi_handle *h, const std::vector<ShotIn> &q, double *img_vp, d
     for (int k = 0; k < 18; k++) *fields[k] = w + (size_t)k * cells;
     a.dbp = h->adj_d.p;
     a.dbs = h->adj_d.p + cells;
+    a.peak = reinterpret_cast<unsigned *>(h->adj_d.p + 2 * cells);
     a.snap = reinterpret_cast<const float *>(b.snap.p);
     a.dz = b.r(R_OBS_Z, nt);
     a.dx = b.r(R_OBS_X, nt);
     if (int rc = wait_observed(h)) return rc;  // the records to back-propagate
     CK(cudaEventRecord(h->ev[2], st));
-    for (int it = nt - 1; it >= 0; it--) launch_adjoint_step(a, it, st);
-    h->launches += 3LL * nt;
+    h->launches += launch_adjoint(a, (long long)b.ntr_tot * nt, st);
     CK(cudaGetLastError());
     CK(cudaEventRecord(h->ev[3], st));
     ImageArgs im{};
@@ -1907,6 +1907,8 @@ int born_adjoint(sfwi_handle *h, const std::vector<ShotIn> &q, double *img_vp, d
     im.nshots = b.nshots;
     im.geo = b.dgeo.p;
     im.dbp = a.dbp;
+    im.peak = a.peak;
+    im.dt = h->dt;
     im.dbs = a.dbs;
     im.vp = b.g(C_VP);
     im.vs = b.g(C_VS);

@@ -170,7 +170,7 @@ void launch_ot_scales(const float *obs_z, const float *obs_x, int nt, int ntr, c
 
 // sfwi_adjoint.cu: the exact adjoint of the Born modelling operator
 struct AdjArgs {
-    int X, P, PS, pml, nt, born_lo;
+    int X, P, PS, pml, nt;
     float dt, dtdx, dtdz, idx, idz;
     const ShotGeo *geo;
     const int *rowshot;  // [X]: the shot of each packed row
@@ -179,16 +179,22 @@ struct AdjArgs {
     // the transposed stencils gather, each [X][P]
     float *avx, *avz, *amx, *amz, *atxx, *atzz, *atxz, *amxx, *amzz, *amxz;
     float *gax, *gbz, *gcz, *gdx, *hax, *hbz, *hdx, *hcz;
-    double *dbp, *dbs;   // adjoints of 2 rho vp dVp and 2 rho vs dVs per window cell
+    // adjoints of 2 rho vp dVp and 2 rho vs dVs per window cell, over dt and in units
+    // set by `peak`: float pairs (sfwi_d2.cuh)
+    float2 *dbp, *dbs;
+    unsigned *peak;  // [2], zero: the largest record and background velocity, as bits
     const float *snap;   // background vx, vz after each step's velocity sweep, [2 it + comp][X][PS]
     const float *dz, *dx;  // the data (records' adjoint), trace-major [ntr][nt]
     const int *rstart, *rtr;  // per packed row: the traces recorded there, rtr[rstart[row] .. rstart[row+1])
 };
-void launch_adjoint_step(const AdjArgs &a, int it, cudaStream_t st);
+// every reverse step (nrec: samples of dz); returns the number of launches
+int launch_adjoint(const AdjArgs &a, long long nrec, cudaStream_t st);
 struct ImageArgs {
     int allnx, allnz, P, pml, nshots;
     const ShotGeo *geo;
-    const double *dbp, *dbs;
+    const float2 *dbp, *dbs;
+    const unsigned *peak;
+    double dt;
     const float *vp, *vs, *rho;
     double *img_vp, *img_vs;
 };

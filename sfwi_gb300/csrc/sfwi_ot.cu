@@ -31,7 +31,7 @@
 // exact in any order, so F_k - G_{m-1} and the search have no rounding but the weights'
 // own (2^-50 at 3000 samples), and equal traces have equal CDFs.  What
 // follows the search (r, its square, the adjoint weights and their sums) is in
-// float pairs of 48 bits (see D2); its cancellation of nearly equal numbers,
+// float pairs of 48 bits (D2, sfwi_d2.cuh); its cancellation of nearly equal numbers,
 // k+1 - T_k, is done in integers before.  Against FP64 the errors are those of the FP64
 // kernel: residuals the same to six digits, misfits at 1e-14.
 // In both the exponential weights are FP32 (expf of the argument rounded to FP32):
@@ -44,6 +44,7 @@
 #include <cudaTypedefs.h>
 #include <mutex>
 
+#include "sfwi_d2.cuh"
 #include "sfwi_launch.h"
 
 namespace sfwi {
@@ -106,33 +107,6 @@ __device__ double block_excl_suffix(double v, double *cs, double *wsum) {
     return r;
 }
 
-// ---------------------------------------------------------------------------
-// float pairs: the unevaluated sum h + l of two floats, |l| <= ulp(h)/2
-// (Dekker 1971, Knuth's two-sum; the product's error term by FMA)
-// ---------------------------------------------------------------------------
-struct D2 {
-    float h, l;
-};
-__device__ __forceinline__ D2 quick2(float a, float b) {  // |a| >= |b| or a = 0
-    const float s = __fadd_rn(a, b);
-    return D2{s, __fadd_rn(b, -__fadd_rn(s, -a))};
-}
-__device__ __forceinline__ D2 sum2(float a, float b) {
-    const float s = __fadd_rn(a, b), t = __fadd_rn(s, -a);
-    return D2{s, __fadd_rn(__fadd_rn(a, -__fadd_rn(s, -t)), __fadd_rn(b, -t))};
-}
-__device__ __forceinline__ D2 operator+(D2 a, D2 b) {  // to 2^-47 (|a| + |b|)
-    const D2 s = sum2(a.h, b.h);
-    return quick2(s.h, __fadd_rn(s.l, __fadd_rn(a.l, b.l)));
-}
-__device__ __forceinline__ D2 operator-(D2 a) { return D2{-a.h, -a.l}; }
-__device__ __forceinline__ D2 operator*(D2 a, D2 b) {
-    const float p = __fmul_rn(a.h, b.h);
-    float e = __fmaf_rn(a.h, b.h, -p);
-    e = __fmaf_rn(a.h, b.l, e);
-    e = __fmaf_rn(a.l, b.h, e);
-    return quick2(p, e);
-}
 __device__ __forceinline__ D2 reciprocal(D2 d) {
     // two terms of the series from an approximate reciprocal of the high part
     const float x = __fdividef(1.f, d.h);
