@@ -703,12 +703,51 @@ std::vector<Strip> march_strips(const ShotGeo &g, int pc, int pml) {
     }
     return v;
 }
-// items of a burst with runs of `rows` rows
-long long burst_count(const sfwi_handle *h, const MarchVariant &w, int rows) {
+// Runs of rows of a burst's items: x-PML rows, other rows of strips that hold
+// z-PML columns, the rest.
+struct BurstRuns {
+    int edge, side, rest;
+};
+// the ends of the runs of a strip
+std::vector<int> burst_cuts(const ShotGeo &g, int pml, const Strip &q, const BurstRuns &r) {
+    const int e = pml + NOP, f = g.nxpml - pml - NOP, inner = q.side > 1.0 ? r.side : r.rest;
+    std::vector<int> cut{NOP};
+    for (int x = NOP; x < g.nxpml - NOP;) {
+        // (whole groups, so that only a strip's last run has a part of one)
+        int len = r.edge;
+        if (x + G_ROWS > e && x < f) len = std::max(std::min(inner, (f - x) / G_ROWS * G_ROWS), G_ROWS);
+        cut.push_back(x = std::min(x + len, g.nxpml - NOP));
+    }
+    return cut;
+}
+long long burst_count(const sfwi_handle *h, const MarchVariant &w, const BurstRuns &r) {
     long long n = 0;
     for (const ShotGeo &g : h->b.geo)
-        n += (long long)march_strips(g, w.ps - 16, h->pml).size() * ((g.nxpml - 2 * NOP + rows - 1) / rows);
+        for (const Strip &q : march_strips(g, w.ps - 16, h->pml)) n += (long long)burst_cuts(g, h->pml, q, r).size() - 1;
     return n;
+}
+// A step of a burst ends with its slowest item, and an item takes as many
+// rounds as its groups need of the four teams of warps, in either half-step:
+// the runs that make the slowest class of items fastest, then all of them, while every
+// item has a slot (one Born shot at 299x151: 6.1 -> 5.4, 7.1 -> 6.6 us against equal
+// runs; at 376x201 7.0 -> 6.9, 7.8 -> 7.7 us)
+BurstRuns burst_runs(const sfwi_handle *h, const MarchVariant &w, int slots) {
+    auto rounds = [](int rows) {
+        const int n = rows / G_ROWS;
+        return (n + 2 + 3) / 4 + (n + 3) / 4 + 0.05 * rows;  // (and its loads)
+    };
+    BurstRuns best{BURST_ROWS, BURST_ROWS, BURST_ROWS};
+    double least = -1, sum = 0;
+    for (int e = G_ROWS; e <= BURST_ROWS; e += G_ROWS)
+        for (int s = G_ROWS; s <= BURST_ROWS; s += G_ROWS)
+            for (int r = G_ROWS; r <= BURST_ROWS; r += G_ROWS) {
+                const double te = MARCH_EDGE * rounds(e), ts = MARCH_SIDE * rounds(s), tr = rounds(r);
+                const double c = std::max({te, ts, tr}), t = te + ts + tr;
+                if (least >= 0 && (c > least || (c == least && t >= sum))) continue;
+                if (burst_count(h, w, BurstRuns{e, s, r}) > slots) continue;
+                best = BurstRuns{e, s, r}, least = c, sum = t;
+            }
+    return best;
 }
 void march_items(const sfwi_handle *h, const MarchVariant &w, int slots, std::vector<MarchItem> &items,
                  std::vector<int> &active) {
@@ -729,9 +768,9 @@ void march_items(const sfwi_handle *h, const MarchVariant &w, int slots, std::ve
         tot.push_back(rows_cost(g, g.nxpml));
     }
     double best = 8, cost = 0;
+    BurstRuns runs{};
     if (burst) {
-        // the shortest runs that still give every slot one item
-        for (best = G_ROWS; best < BURST_ROWS && burst_count(h, w, (int)best) > slots;) best += G_ROWS;
+        runs = burst_runs(h, w, slots);
     } else {
         for (double len = 4; len <= 1024; len *= 1.02) {
             long long n = 0;
@@ -758,8 +797,7 @@ void march_items(const sfwi_handle *h, const MarchVariant &w, int slots, std::ve
             int x = NOP;
             cut[q].push_back(x);
             if (burst) {
-                while (x < g.nxpml - NOP) cut[q].push_back(x += (int)best);
-                cut[q].back() = g.nxpml - NOP;
+                cut[q] = burst_cuts(g, pml, st[s][q], runs);
                 most = std::max(most, cut[q].size());
                 continue;
             }
@@ -844,7 +882,7 @@ void plan_march(sfwi_handle *h, bool forward_only) {
     }
     const long long per_sm = cells / std::max(h->nsm, 1);
     if (per_sm < MARCH_MIN_CELLS) return;
-    const bool one_wave = burst_count(h, *march_burst(), BURST_ROWS) <= h->nsm, large = per_sm >= MARCH_LARGE_CELLS;
+    const bool one_wave = burst_count(h, *march_burst(), {BURST_ROWS, BURST_ROWS, BURST_ROWS}) <= h->nsm, large = per_sm >= MARCH_LARGE_CELLS;
     const bool taken = !forward_only && snap;  // snapshots are stored
     const int every = taken ? h->snap_every : INT_MAX;
     const bool fits = one_wave || per_sm >= MARCH_ANY_CELLS || 10 * cells >= 7 * room;
