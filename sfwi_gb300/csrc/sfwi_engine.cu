@@ -846,8 +846,8 @@ void no_march(Batch &b) {
 }
 // Decide whether the batch runs whole steps per launch, and plan it.  Per
 // step, sweeps -> whole step, 152 SMs (stage 1 / Born forward; backward):
-//   one wave of bursts, every SM at most one item (376x201, one shot): 8.3 -> 5.7 /
-//     9.8 -> 7.1; 11.1 -> 8.2 us.  Two waves (two shots) lose: 10.2 -> 10.4,
+//   one wave of bursts, every SM at most one item (376x201, one shot): 8.3 -> 5.0 /
+//     9.8 -> 6.3; 11.1 -> 6.9 us.  Two waves (two shots) lose: 10.2 -> 10.4,
 //     13.5 -> 15.0 us.
 //   forward march, larger batches: 2 shots 10.2 -> 8.8 / 12.0 -> 11.2, 4 shots 15.3 -> 12.2 /
 //     18.8 -> 14.4, 12 shots 26.0 -> 23.9 / 36.0 -> 35.0, 38 shots 67 -> 62 / 107 -> 92 us.

@@ -390,7 +390,7 @@ struct FwdBody {
                     load_damp(a, o, xd, fx[i], fz[i]);
                     mx[i] = ldl<PAIR>(in.mvx + o * E);
                     mz[i] = ldl<PAIR>(in.mvz + o * E);
-                    if (r.lx + G < g.nxpml) {
+                    if (!C::BURST && r.lx + G < g.nxpml) {
                         // the next group's, while this one is computed
                         const size_t n = o + G * g.P;
                         prefetch_l2(a.fz + 2 * n);
@@ -575,7 +575,7 @@ struct FwdBody {
                     mxx[i] = ldl<PAIR>(in.mtxx + o * E);
                     mzz[i] = ldl<PAIR>(in.mtzz + o * E);
                     mxz[i] = ldl<PAIR>(in.mtxz + o * E);
-                    if (r.lx + G < g.nxpml) {
+                    if (!C::BURST && r.lx + G < g.nxpml) {
                         const size_t n = o + G * g.P;
                         prefetch_l2(in.mtxx + n * E);
                         prefetch_l2(in.mtzz + n * E);
@@ -776,7 +776,8 @@ __global__ void __launch_bounds__((FwdCfg<PS, PAIR, false>::NT), (FwdCfg<PS, PAI
 
 // The groups of a short item all at once.  Bound by latency: a launch, the
 // loads, two half-steps of one or two groups a warp.  One stage-1 shot at 376x201
-// 8.3 -> 5.7 us a step, at 149x83 7.7 -> 4.7 us (Born 9.1 -> 4.7 us).
+// 8.3 -> 5.0 us a step, at 149x83 7.7 -> 4.4 us (Born 9.1 -> 4.4 us).  No prefetches: the
+// next group is at work next door, and they cost 0.4 us a step.
 template <int PS, bool PAIR, bool SNAP>
 __global__ void __launch_bounds__((FwdCfg<PS, PAIR, true>::NT), 1)
     k_burst_fwd(const __grid_constant__ MarchArgs a, const __grid_constant__ MarchMaps tm, int it) {
@@ -1068,7 +1069,7 @@ struct BwdBody {
                         mxx[i] = ldl<PAIR>(in.mtxx + o * E);
                         mzz[i] = ldl<PAIR>(in.mtzz + o * E);
                     }
-                    if (r.lx + G < g.nxpml) {
+                    if (!C::BURST && r.lx + G < g.nxpml) {
                         // the next group's, while this one is computed
                         const size_t n = o + G * g.P;
                         prefetch_l2(a.fz + 2 * n);
@@ -1084,7 +1085,7 @@ struct BwdBody {
             if (PAIR && image_row<F>(r) && (sc.is(Cols::IM0 | Cols::IM1))) {
                 gl[i] = ld2g(p.glam + o);
                 gm[i] = ld2g(p.gmu + o);
-                if (r.lx + G < g.nxpml) {
+                if (!C::BURST && r.lx + G < g.nxpml) {
                     prefetch_l2(p.glam + o + G * g.P);
                     prefetch_l2(p.gmu + o + G * g.P);
                 }
@@ -1229,7 +1230,7 @@ struct BwdBody {
                     load_damp(a, o, xd, fx[i], fz[i]);
                     mx[i] = ldl<PAIR>(in.mvx + o * E);
                     mz[i] = ldl<PAIR>(in.mvz + o * E);
-                    if (r.lx + G < g.nxpml) {
+                    if (!C::BURST && r.lx + G < g.nxpml) {
                         prefetch_l2(in.mvx + (o + G * g.P) * E);
                         prefetch_l2(in.mvz + (o + G * g.P) * E);
                     }
@@ -1238,7 +1239,7 @@ struct BwdBody {
             if (PAIR && image_row<F>(r) && (vc.is(Cols::IM0 | Cols::IM1))) {
                 il[i] = ld2g(p.illum + o);
                 if (RHO) gr[i] = ld2g(p.grho + o);
-                if (r.lx + G < g.nxpml) {
+                if (!C::BURST && r.lx + G < g.nxpml) {
                     prefetch_l2(p.illum + o + G * g.P);
                     if (RHO) prefetch_l2(p.grho + o + G * g.P);
                 }
@@ -1413,7 +1414,7 @@ __global__ void __launch_bounds__((BwdCfg<PS, PAIR, false>::NT), (BwdCfg<PS, PAI
     }
 }
 
-// One shot at 376x201 11.1 -> 7.8 us a step, at 149x83 10.4 -> 5.5 us.  The strips and
+// One shot at 376x201 11.1 -> 6.9 us a step, at 149x83 10.4 -> 5.1 us.  The strips and
 // residuals are fetched while the loads are on their way: read row by row after
 // them they cost 6 us.
 template <int PS, bool PAIR, bool RHO>
