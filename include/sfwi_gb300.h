@@ -349,9 +349,10 @@ int sfwi_set_source(sfwi_handle *h, int kind);
  * batches that gain from it run whole time steps per launch (sfwi_march.cu, chosen by
  * the batch's size; it takes a second copy of the wavefields where memory
  * is plentiful), with the same results bit for bit; other batches run the
- * sweeps.  Until a shape is selected (here or by sfwi_autotune) each batch gets SFWI_TILE_16x32, or
- * SFWI_TILE_8x32_2CELL_3STAGE when its 16x32 tiles would give fewer than four
- * to each of the device's CTA slots (small batches).  A batch already on
+ * sweeps.  Until a shape is selected (here or by sfwi_autotune) each batch
+ * gets SFWI_TILE_16x32, or, when its 16x32 tiles would give fewer than four to
+ * each of the device's CTA slots, SFWI_TILE_16x32_2CELL (fewer than 1.75:
+ * SFWI_TILE_8x32_2CELL_3STAGE).  A batch already on
  * the device is re-tiled.  Results do not depend on the shape: they are
  * bit-identical, since every cell takes the same update (split where the cell
  * is damped, plain elsewhere, whatever its tile holds), reads the same values

@@ -379,8 +379,8 @@ int encode_grid_map(CUtensorMap *m, float *base, int P, int X, int bz, int bx, i
     const cuuint64_t strides[2] = {(cuuint64_t)P * es, (cuuint64_t)P * X * es};
     const cuuint32_t box[3] = {(cuuint32_t)bz, (cuuint32_t)bx, (cuuint32_t)depth};
     const cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = enc(m, pairs ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box, estr,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+    CUresult r = enc(m, pairs ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims,
+                     strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(SFWI_E_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
     return SFWI_OK;
@@ -434,11 +434,11 @@ const TileVariant *tile_variant(int shape) {
 }
 
 // Default tile shape for a batch: the 16x32 tiles when they give every CTA
-// slot (2 per SM) at least four tiles, else 8x32 tiles with two cells per
+// slot (2 per SM) at least four tiles; the same with two cells a thread from
+// 1.75 tiles a slot (backward steps of three, four shots at 376x201 17.2 -> 16.2, 21.2 -> 19.2 us
+// against the next, of six 24.6 -> 24.4 against the last); else 8x32 tiles with two cells per
 // thread and three pipeline stages, which double the tiles of a small batch
-// and keep more of them in flight (one 376x201 shot: 196 16x32 tiles for 304
-// slots; a step is 20 % faster on those tiles; a 38-shot batch is 14 %
-// faster on 16x32).  sfwi_set_tile_shape or sfwi_autotune replace the rule.
+// and keep more of them in flight (two shots 15.3 -> 13.5 us).  sfwi_set_tile_shape or sfwi_autotune replace the rule.
 // padded depth of a shot: its own model's in a several-model batch
 int shot_nzpml(const sfwi_handle *h, const ShotIn &in) {
     return in.req >= 0 ? h->models[in.req].allnz + 2 * h->pml : h->nzpml;
@@ -450,7 +450,10 @@ void pick_tile_shape(sfwi_handle *h, const std::vector<ShotIn> &shots) {
         const int zt = (shot_nzpml(h, in) - 2 * NOP + 31) / 32;
         tiles += (long long)((in.nx + 2 * h->pml - 2 * NOP + 15) / 16) * zt;
     }
-    h->tv = tile_variant(tiles < 4LL * 2 * std::max(h->nsm, 1) ? SFWI_TILE_8x32_2CELL_3STAGE : SFWI_TILE_16x32);
+    const long long slots = 2LL * std::max(h->nsm, 1);
+    h->tv = tile_variant(4 * tiles < 7 * slots ? SFWI_TILE_8x32_2CELL_3STAGE
+                         : tiles < 4 * slots   ? SFWI_TILE_16x32_2CELL
+                                               : SFWI_TILE_16x32);
 }
 
 // Tiles of one axis of length n (with PML width pml) that start at `start`
@@ -723,7 +726,8 @@ std::vector<int> burst_cuts(const ShotGeo &g, int pml, const Strip &q, const Bur
 long long burst_count(const sfwi_handle *h, const MarchVariant &w, const BurstRuns &r) {
     long long n = 0;
     for (const ShotGeo &g : h->b.geo)
-        for (const Strip &q : march_strips(g, w.ps - 16, h->pml)) n += (long long)burst_cuts(g, h->pml, q, r).size() - 1;
+        for (const Strip &q : march_strips(g, w.ps - 16, h->pml))
+            n += (long long)burst_cuts(g, h->pml, q, r).size() - 1;
     return n;
 }
 // A step of a burst ends with its slowest item, and an item takes as many
@@ -851,13 +855,18 @@ void no_march(Batch &b) {
 //     13.5 -> 15.0 us.
 //   forward march, larger batches: 2 shots 10.2 -> 8.8 / 12.0 -> 11.2, 4 shots 15.3 -> 12.2 /
 //     18.8 -> 14.4, 12 shots 26.0 -> 23.9 / 36.0 -> 35.0, 38 shots 67 -> 62 / 107 -> 92 us.
-//     Below 2,000 cells an SM strips that are far from full lose (five shots of 153
-//     columns, two strips of 80: 9.4 -> 10.4; three of 183, two of 92: 9.0 -> 8.3).  Born
+//     Below 1,150 cells an SM the sweeps' smaller tiles keep up (eight shots at 149x83 9.2 /
+//     11.2 -> 9.1 / 11.5), below 2,000 strips that are far from full lose (five shots of 153
+//     columns, two strips of 80: 9.4 -> 10.4; three of 183, two of 92: 9.0 -> 8.3), and
+//     above 9,000 plain fields without snapshots in strips less than 95 % full (20
+//     shots of 333 columns, three strips of 112: 51.2 -> 55.4, 10 shots 29.7 -> 29.9, 6
+//     shots 22.1 -> 20.1).  Born
 //     between 8,000 and 15,000 cells an SM it depends on how the runs divide (ten
 //     shots at 401x301: 42.7 -> 44.2, uneven apertures 56.5 -> 55.7 us): sweeps
 //   backward march, pairs: the fill of the rings and the recomputed rim are a
 //     constant cost per item, so it pays from about 15,000 cells an SM (7,500:
-//     41.1 -> 43.6, 13,500: 65.2 -> 69.0, 15,000: 78.7 -> 75.2, 24,000: 121 -> 111 us)
+//     41.1 -> 43.6, 13,500: 65.2 -> 69.0, 15,000: 78.7 -> 75.2, 24,000: 121 -> 111 us) in
+//     nearly full strips (19,000 in strips of 112: 98.5 -> 102)
 //   snapshots are launches of their own here and part of the sweeps there.  Nine
 //     shots at 376x201, every 1, 2, 4 steps: adjoint 23.9 -> 30.2, 22.5 -> 23.9,
 //     21.7 -> 20.5; Born forward 29.4 -> 33.0, 28.8 -> 30.2, 28.4 -> 28.8 (38 shots: as
@@ -865,7 +874,8 @@ void no_march(Batch &b) {
 //     shots, in 16 bits 25.2 -> 21.5, 23.2 -> 20.2, 22.4 -> 19.2 us
 // Grids of less than 64 cells an SM stay with the sweeps: such a step is all
 // launch latency, and the launch counts of the golden cases are the sweeps'.
-constexpr long long MARCH_MIN_CELLS = 64, MARCH_ANY_CELLS = 2000, MARCH_MID_CELLS = 8000, MARCH_LARGE_CELLS = 15000;
+constexpr long long MARCH_MIN_CELLS = 64, MARCH_FEW_CELLS = 1150, MARCH_ANY_CELLS = 2000, MARCH_MID_CELLS = 8000,
+                    MARCH_PLAIN_CELLS = 9000, MARCH_LARGE_CELLS = 15000;
 constexpr int MARCH_SNAP_EVERY = 4;
 void plan_march(sfwi_handle *h, bool forward_only) {
     Batch &b = h->b;
@@ -882,14 +892,16 @@ void plan_march(sfwi_handle *h, bool forward_only) {
     }
     const long long per_sm = cells / std::max(h->nsm, 1);
     if (per_sm < MARCH_MIN_CELLS) return;
-    const bool one_wave = burst_count(h, *march_burst(), {BURST_ROWS, BURST_ROWS, BURST_ROWS}) <= h->nsm, large = per_sm >= MARCH_LARGE_CELLS;
+    const bool one_wave = burst_count(h, *march_burst(), {BURST_ROWS, BURST_ROWS, BURST_ROWS}) <= h->nsm;
+    const bool large = per_sm >= MARCH_LARGE_CELLS;
     const bool taken = !forward_only && snap;  // snapshots are stored
     const int every = taken ? h->snap_every : INT_MAX;
-    const bool fits = one_wave || per_sm >= MARCH_ANY_CELLS || 10 * cells >= 7 * room;
-    const bool fwd = !fits ? false
+    const bool fits = one_wave || per_sm >= MARCH_ANY_CELLS || (per_sm >= MARCH_FEW_CELLS && 10 * cells >= 7 * room);
+    const bool full = 20 * cells >= 19 * room;  // strips nearly full
+    const bool fwd = !fits || (!born && !full && !taken && per_sm > MARCH_PLAIN_CELLS) ? false
                      : born ? (per_sm < MARCH_MID_CELLS || large) && every >= MARCH_SNAP_EVERY
                             : every > 1 || h->snap_fmt != SNAP_F32;
-    const bool bwd = taken ? every >= MARCH_SNAP_EVERY : one_wave || large;
+    const bool bwd = taken ? every >= MARCH_SNAP_EVERY : one_wave || (large && full);
     const MarchVariant *way = one_wave ? march_burst() : march_wide();
     if (fwd) b.way[0] = way;
     if (bwd && !forward_only) b.way[1] = way;
@@ -921,7 +933,8 @@ int upload_march(sfwi_handle *h, bool forward_only) {
     const size_t nf = b.items[0].size(), nb = b.items[1].size();
     CK(b.ditems.ensure(nf + nb));
     if (nf) CK(cudaMemcpyAsync(b.ditems.p, b.items[0].data(), nf * sizeof(MarchItem), cudaMemcpyHostToDevice, h->st));
-    if (nb) CK(cudaMemcpyAsync(b.ditems.p + nf, b.items[1].data(), nb * sizeof(MarchItem), cudaMemcpyHostToDevice, h->st));
+    if (nb)
+        CK(cudaMemcpyAsync(b.ditems.p + nf, b.items[1].data(), nb * sizeof(MarchItem), cudaMemcpyHostToDevice, h->st));
     for (int c = 0; c < 2; c++)
         for (int back = 0; back < 2; back++) {
             if (!b.way[back]) continue;
@@ -933,7 +946,8 @@ int upload_march(sfwi_handle *h, bool forward_only) {
             struct {
                 CUtensorMap *map;
                 int cols, depth;
-            } want[] = {{&m.view3, ps, 3}, {&m.view2, ps, 2}, {&m.rim3, ps - 8, 3}, {&m.rim2, ps - 8, 2}, {&m.core2, ps - 16, 2}};
+            } want[] = {{&m.view3, ps, 3}, {&m.view2, ps, 2}, {&m.rim3, ps - 8, 3}, {&m.rim2, ps - 8, 2},
+                        {&m.core2, ps - 16, 2}};
             for (auto &w : want)
                 if (int rc = encode_grid_map(w.map, base, b.P, b.X, w.cols, 4, w.depth, na, pairs)) return rc;
             struct {

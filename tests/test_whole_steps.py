@@ -71,10 +71,10 @@ def _run(stage, nx, nz, pml, nshots, nt, option, sweeps):
     (1, 201, 190, 11, 6, 33, "snap1 f16"),
     (2, 201, 187, 11, 6, 45, "snap5 f32"),
     (1, 333, 140, 11, 4, 45, "snap4 bf16"),
-    (1, 401, 301, 13, 20, 61, "rho"),
-    (2, 399, 301, 13, 20, 60, "rho"),
-    (1, 499, 233, 20, 18, 60, "lengths"),
-    (1, 401, 301, 13, 19, 61, "host"),
+    (1, 401, 331, 13, 20, 61, "rho"),
+    (2, 399, 331, 13, 20, 60, "rho"),
+    (1, 499, 205, 20, 20, 60, "lengths"),
+    (1, 401, 331, 13, 19, 61, "host"),
 ])
 def test_whole_steps_give_the_sweeps_bits(stage, nx, nz, pml, nshots, nt, option):
     a, few = _run(stage, nx, nz, pml, nshots, nt, option, False)
