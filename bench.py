@@ -82,6 +82,15 @@ KERNEL_BYTES = {
     "k_bwd_s_snap<bf16>": 32 + (4 + 24) / 4,
     "k_bwd_s_snap<f32>": 32 + (8 + 24) / 4,
     "k_bwd_v_snap": 40,    # read sigma_adj(3) + lam, mu, 1/rho; RMW v_adj(2)
+    # whole steps in one launch: every field read and written once a step
+    "k_march_fwd": 52,        # RMW v(2), sigma(3); read lam, mu, 1/rho
+    "k_march_fwd<born>": 100,  # RMW v(2), sigma(3), v_s(2), sigma_s(3); read lam, mu, 1/rho, bp, bs
+    "k_march_bwd": 116,       # RMW v(2), sigma(3), v_adj(2), sigma_adj(3), G_lam, G_mu, illum; read lam, mu, 1/rho
+    # RMW v_adj(2), sigma_adj(3); read lam, mu, 1/rho; at 1 launch in 4 the imaging kernel's
+    # snapshot (2 x 2 or 2 x 4 B), sigma_adj(3) and RMW G_lam, G_mu, illum
+    "k_march_bwd<f16>": 52 + (4 + 12 + 24) / 4,
+    "k_march_bwd<bf16>": 52 + (4 + 12 + 24) / 4,
+    "k_march_bwd<f32>": 52 + (8 + 12 + 24) / 4,
 }
 # algorithmic bytes per padded cell per time step of a Born shot-gradient:
 # forward 72 + reconstruction 72 + adjoint 72 + imaging 32 + Born add-on 80
@@ -442,6 +451,7 @@ def measure(w, args, steps, warmup, plain_shots, pg=None, ws=1, rank=0, clocks=N
     if w.get("rho_grad"):
         fd.set_density_gradient(True)
         kbytes["k_bwd_v"] += 8  # the density kernel's accumulator, read and written
+        kbytes["k_march_bwd"] += 8
 
     def enqueue(d, i):
         b = mine[i]  # the survey shot whose observed records these are
@@ -523,6 +533,12 @@ def measure(w, args, steps, warmup, plain_shots, pg=None, ws=1, rank=0, clocks=N
 
     # per-kernel average launch durations (CUDA events on the engine stream)
     kt = fd.time_kernels(reps=20)
+    if launches < 2.9 * nt * steps:
+        # both directions ran whole steps per launch, not the four sweeps
+        # that were just timed: a step's time from its phase of the passes
+        snap = "<%s>" % w["snap"][1] if w.get("snap") else ""
+        kt = {"k_march_fwd<born>" if fd.stage == 2 else "k_march_fwd": float(np.mean(fwd_ms)) / nt,
+              "k_march_bwd" + snap: float(np.mean(bwd_ms)) / nt}
     peak, peak_kind = measured_peak_hbm()
     cells = sum((d["nx"] + 2 * pml) * nzpml for d in shots)
     roof, fracs = None, None
@@ -533,7 +549,7 @@ def measure(w, args, steps, warmup, plain_shots, pg=None, ws=1, rank=0, clocks=N
         tpc = traffic_per_cell(dom)
         roof = {"bound": "hbm", "kernel": dom, "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                 "frac": round(achieved / peak, 4), "traffic": round(tpc * cells) if tpc else None,
-                "traffic_note": "DRAM bytes per launch: ncu capture of a 16-shot launch scaled by cells",
+                "traffic_note": "DRAM bytes per launch: ncu capture of a 16-shot (whole steps: 38-shot) launch scaled by cells",
                 # the DRAM side of the same launch: measured bytes over the event time
                 "dram_achieved": round(tpc * cells / (kt[dom] / 1000.0) / 1e9, 1) if tpc else None,
                 "alg_bytes_per_launch": kbytes[dom] * cells, "peak_source": peak_kind,
