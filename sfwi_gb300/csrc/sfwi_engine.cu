@@ -856,13 +856,16 @@ void no_march(Batch &b) {
 //   forward march, larger batches: 2 shots 10.2 -> 8.8 / 12.0 -> 11.2, 4 shots 15.3 -> 12.2 /
 //     18.8 -> 14.4, 12 shots 26.0 -> 23.9 / 36.0 -> 35.0, 38 shots 67 -> 62 / 107 -> 92 us.
 //     Below 1,150 cells an SM the sweeps' smaller tiles keep up (eight shots at 149x83 9.2 /
-//     11.2 -> 9.1 / 11.5), below 2,000 strips that are far from full lose (five shots of 153
-//     columns, two strips of 80: 9.4 -> 10.4; three of 183, two of 92: 9.0 -> 8.3), and
-//     above 9,000 plain fields without snapshots in strips less than 95 % full (20
-//     shots of 333 columns, three strips of 112: 51.2 -> 55.4, 10 shots 29.7 -> 29.9, 6
-//     shots 22.1 -> 20.1).  Born
-//     between 8,000 and 15,000 cells an SM it depends on how the runs divide (ten
-//     shots at 401x301: 42.7 -> 44.2, uneven apertures 56.5 -> 55.7 us): sweeps
+//     11.2 -> 9.1 / 11.5).  Above, plain fields lose where much of the grid is PML, the
+//     marches' slow form (62x63 at PML 20, 43 shots: 12.3 -> 15.0; 150x190, 13 shots 14.1 -> 15.4;
+//     250x215 in strips 69 % full, 8 shots 14.0 -> 14.5; against 300x160 at PML 11, 10 shots
+//     14.5 -> 13.5), and above 9,000 cells an SM, without snapshots, in strips less
+//     than 95 % full (20 shots of 333 columns, three strips of 112: 51.2 -> 55.4, 6 shots
+//     22.1 -> 20.1).  Born fields gain up to 3,500 cells an SM whatever the strips (300x120,
+//     63 % full, 8 shots 17.1 -> 15.9, 11 shots 21.5 -> 21.5, 15 shots 25.6 -> 27.5),
+//     above that in one strip (400x80, 30 shots 40.3 -> 35.6) or full ones; between 8,000 and 15,000 it depends on
+//     how the runs divide (ten shots at 401x301: 42.7 -> 44.2, uneven apertures
+//     56.5 -> 55.7 us): sweeps
 //   backward march, pairs: the fill of the rings and the recomputed rim are a
 //     constant cost per item, so it pays from about 15,000 cells an SM (7,500:
 //     41.1 -> 43.6, 13,500: 65.2 -> 69.0, 15,000: 78.7 -> 75.2, 24,000: 121 -> 111 us) in
@@ -874,7 +877,7 @@ void no_march(Batch &b) {
 //     shots, in 16 bits 25.2 -> 21.5, 23.2 -> 20.2, 22.4 -> 19.2 us
 // Grids of less than 64 cells an SM stay with the sweeps: such a step is all
 // launch latency, and the launch counts of the golden cases are the sweeps'.
-constexpr long long MARCH_MIN_CELLS = 64, MARCH_FEW_CELLS = 1150, MARCH_ANY_CELLS = 2000, MARCH_MID_CELLS = 8000,
+constexpr long long MARCH_MIN_CELLS = 64, MARCH_FEW_CELLS = 1150, MARCH_ANY_CELLS = 3500, MARCH_MID_CELLS = 8000,
                     MARCH_PLAIN_CELLS = 9000, MARCH_LARGE_CELLS = 15000;
 constexpr int MARCH_SNAP_EVERY = 4;
 void plan_march(sfwi_handle *h, bool forward_only) {
@@ -883,24 +886,34 @@ void plan_march(sfwi_handle *h, bool forward_only) {
     // (a cell's offset is computed in 32 bits)
     if (!h->march_ok || (long long)b.X * b.P >= (1LL << 31)) return;
     const bool born = h->stage == 2, snap = h->snap_every > 0;
-    long long cells = 0, room = 0;  // room: cells of full strips
+    long long cells = 0, room = 0, inner = 0;  // updated; of full strips; outside the PML
+    bool one_strip = true;
     const int pc = march_wide()->ps - 16;
     for (const ShotGeo &g : b.geo) {
         const int rows = g.nxpml - 2 * NOP, cols = g.nzpml - 2 * NOP;
         cells += (long long)rows * cols;
         room += (long long)rows * ((cols + pc - 1) / pc * pc);
+        inner += (long long)(g.nxpml - 2 * h->pml) * (g.nzpml - 2 * h->pml);
+        one_strip &= cols <= pc;
     }
     const long long per_sm = cells / std::max(h->nsm, 1);
     if (per_sm < MARCH_MIN_CELLS) return;
-    const bool one_wave = burst_count(h, *march_burst(), {BURST_ROWS, BURST_ROWS, BURST_ROWS}) <= h->nsm;
+    // (an item has BURST_ROWS rows of a strip at most: most batches need no count)
+    const bool one_wave = per_sm <= (long long)BURST_ROWS * (march_burst()->ps - 16) &&
+                          burst_count(h, *march_burst(), {BURST_ROWS, BURST_ROWS, BURST_ROWS}) <= h->nsm;
     const bool large = per_sm >= MARCH_LARGE_CELLS;
     const bool taken = !forward_only && snap;  // snapshots are stored
     const int every = taken ? h->snap_every : INT_MAX;
-    const bool fits = one_wave || per_sm >= MARCH_ANY_CELLS || (per_sm >= MARCH_FEW_CELLS && 10 * cells >= 7 * room);
-    const bool full = 20 * cells >= 19 * room;  // strips nearly full
-    const bool fwd = !fits || (!born && !full && !taken && per_sm > MARCH_PLAIN_CELLS) ? false
-                     : born ? (per_sm < MARCH_MID_CELLS || large) && every >= MARCH_SNAP_EVERY
-                            : every > 1 || h->snap_fmt != SNAP_F32;
+    const bool full = 20 * cells >= 19 * room, nearly = 10 * cells >= 9 * room;  // strips full to 95, 90 %
+    // cells outside the PML, of all and of full strips' room
+    const bool plain = 100 * inner >= 74 * cells && 100 * inner >= 55 * room;
+    const bool fwd = one_wave ? (born ? every >= MARCH_SNAP_EVERY : every > 1 || h->snap_fmt != SNAP_F32)
+                     : per_sm < MARCH_FEW_CELLS ? false
+                     : born ? every >= MARCH_SNAP_EVERY &&
+                                  (per_sm < MARCH_ANY_CELLS || (per_sm < MARCH_MID_CELLS && (one_strip || full)) ||
+                                   (large && (one_strip || nearly)))
+                            : (every > 1 || h->snap_fmt != SNAP_F32) && plain &&
+                                  (full || taken || per_sm <= MARCH_PLAIN_CELLS);
     const bool bwd = taken ? every >= MARCH_SNAP_EVERY : one_wave || (large && full);
     const MarchVariant *way = one_wave ? march_burst() : march_wide();
     if (fwd) b.way[0] = way;
