@@ -134,7 +134,8 @@ __global__ void k_adj_peaks(const __grid_constant__ AdjArgs a, long long nrec) {
             v = fmaxf(v, fmaxf(fmaxf(fabsf(w.x), fabsf(w.y)), fmaxf(fabsf(w.z), fabsf(w.w))));
         }
     }
-    const unsigned r = __reduce_max_sync(0xffffffffu, __float_as_uint(m)), s = __reduce_max_sync(0xffffffffu, __float_as_uint(v));
+    const unsigned r = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+    const unsigned s = __reduce_max_sync(0xffffffffu, __float_as_uint(v));
     if ((threadIdx.x & 31) == 0) {
         atomicMax(a.peak, r);
         atomicMax(a.peak + 1, s);

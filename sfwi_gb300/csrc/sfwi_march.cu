@@ -66,8 +66,7 @@ __device__ __forceinline__ float *smem() {
 // ---------------------------------------------------------------------------
 template <bool PAIR>
 struct Lanes {
-    static constexpr int N = PAIR ? 2 : 1;  // lanes
-    static constexpr int E = PAIR ? 2 : 1;  // floats of a cell
+    static constexpr int N = PAIR ? 2 : 1;
     float2 v[N];
     __device__ __forceinline__ float2 &operator[](int i) { return v[i]; }
     __device__ __forceinline__ const float2 &operator[](int i) const { return v[i]; }
@@ -350,7 +349,8 @@ struct FwdBody {
         vc = cols_at(g, g.z0 - NOP, 2 * cp, C::PV, g.z0 + g.zw + NOP);
         sc = cols_at(g, g.z0, 2 * cp, C::PC, g.z0 + g.zw);
         const int d0 = vc.z - (g.pml - NOP), d1 = vc.z - (g.nzpml - g.pml - NOP);
-        strip_z = __any_sync(0xffffffffu, vc.is(Cols::OWN) && ((d0 >= -1 && d0 < 2 * NOP) || (d1 >= -1 && d1 < 2 * NOP)));
+        strip_z = __any_sync(0xffffffffu, vc.is(Cols::OWN) && ((d0 >= -1 && d0 < 2 * NOP) ||
+                                                               (d1 >= -1 && d1 < 2 * NOP)));
         const bool src = im.m.flags & MARCH_SOURCE;
         auto holds = [](int z, int w) { return w == z || w == z + 1; };
         special(vc, strip_z || holds(vc.z, im.m.g.igz) || (src && holds(vc.z, im.m.g.isz)));
@@ -666,7 +666,8 @@ struct FwdBody {
 #pragma unroll
                 for (int c = 0; c < 3; c++)
 #pragma unroll
-                    for (int l = 0; l < N; l++) n[c][l] = pick<PAIR>(l, true, sc.is(Cols::OK1), n[c][l], make_float2(0.f, 0.f));
+                    for (int l = 0; l < N; l++)
+                        n[c][l] = pick<PAIR>(l, true, sc.is(Cols::OK1), n[c][l], make_float2(0.f, 0.f));
             }
             if (own) {
                 stl<PAIR>(out.txx + o * E, n[0]);

@@ -485,7 +485,9 @@ __global__ void __maxnreg__(56) k_ot(OtArgs a, int run) {
         block_sum2(sx, sy, ws[1]);
         if (threadIdx.x == 0) {
             // (a margin for the rounding of these sums)
-            auto room = [&](float t) { return t > 0.f ? min(max(all_ones, 62 - (ilogbf(1.01f * t) + 1)), 62) : all_ones; };
+            auto room = [&](float t) {
+                return t > 0.f ? min(max(all_ones, 62 - (ilogbf(1.01f * t) + 1)), 62) : all_ones;
+            };
             tc.bc = room(sx.h), tc.bo = room(sy.h);
         }
         __syncthreads();
