@@ -308,6 +308,12 @@ int sfwi_debug_grid_shape(sfwi_handle *h, int *X, int *P, int *narrays, int *nst
 int sfwi_debug_tile_grid(int pml, int nzpml, int tx, int tz, const int *nxpml, int nshots, int *z_start,
                          int *x_start, int *tiles, int *frame_tiles);
 int sfwi_debug_read_grid(sfwi_handle *h, int array, float *dst);
+/* Debugging: how the last run's batch took its forward and backward time
+ * steps (a forward-only run: backward SFWI_STEPS_SWEEPS). */
+#define SFWI_STEPS_SWEEPS 0 /* a velocity and a stress sweep, one launch each */
+#define SFWI_STEPS_MARCH 1  /* one launch a step, its items row group by row group */
+#define SFWI_STEPS_BURST 2  /* one launch a step, its items all at once */
+int sfwi_debug_steps(sfwi_handle *h, int *forward, int *backward);
 
 /* Failure path of the device-side waits, without a fault: runs the tile
  * pipeline of the last batch with a producer that stages nothing and a wait

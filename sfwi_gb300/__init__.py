@@ -366,6 +366,14 @@ class FD2DGPU_ELASTIC:
             _lib.check(_lib.load().sfwi_debug_read_grid(self._h, a, _fp(out[a])))
         return out, ns.value
 
+    def debug_steps(self):
+        """How the last run's batch took its (forward, backward) time steps:
+        "sweeps", or whole steps per launch as a "march" or a "burst"."""
+        d = (C.c_int * 2)()
+        _lib.check(_lib.load().sfwi_debug_steps(self._h, C.cast(d, C.POINTER(C.c_int)),
+                                                C.cast(C.byref(d, C.sizeof(C.c_int)), C.POINTER(C.c_int))))
+        return tuple(("sweeps", "march", "burst")[k] for k in d)
+
     def wait_selftest(self, tries=4096):
         """Make the device-side pipeline waits of the last batch's tile
         pipeline run out (bounded, no fault); raises SfwiError carrying the

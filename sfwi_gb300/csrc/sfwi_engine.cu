@@ -2772,6 +2772,17 @@ int sfwi_debug_read_grid(sfwi_handle *h, int array, float *dst) {
     return SFWI_OK;
 }
 
+int sfwi_debug_steps(sfwi_handle *h, int *forward, int *backward) {
+    if (int rc = check(h)) return rc;
+    if (!h->b.ready) return fail(SFWI_E_STATE, "no batch on the device");
+    auto kind = [](const MarchVariant *w) {
+        return !w ? SFWI_STEPS_SWEEPS : w->burst ? SFWI_STEPS_BURST : SFWI_STEPS_MARCH;
+    };
+    if (forward) *forward = kind(h->b.way[0]);
+    if (backward) *backward = kind(h->b.way[1]);
+    return SFWI_OK;
+}
+
 int sfwi_wait_selftest(sfwi_handle *h, unsigned tries) {
     if (int rc = check(h)) return rc;
     if (tries < 1 || tries > PIPE_WAIT_LIMIT) return fail(SFWI_E_ARG, "tries must be in 1..%u", PIPE_WAIT_LIMIT);
