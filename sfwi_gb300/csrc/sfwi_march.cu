@@ -355,6 +355,9 @@ struct FwdBody {
         auto holds = [](int z, int w) { return w == z || w == z + 1; };
         special(vc, strip_z || holds(vc.z, im.m.g.igz) || (src && holds(vc.z, im.m.g.isz)));
         special(sc, src && holds(sc.z, im.m.g.isz));
+        // a vertical force below the update region enters the stress half-step's view
+        if (src && a.p.src_kind == SRC_VZ_FORCE && __any_sync(0xffffffffu, holds(vc.z, im.m.g.isz)))
+            vc.f &= ~Cols::NONE;
     }
 
     // the thread's rows of group k: new velocities into the ring (zero outside
