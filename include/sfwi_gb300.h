@@ -291,7 +291,9 @@ int sfwi_last_timing(sfwi_handle *h, float *fwd_ms, float *bwd_ms, float *other_
  * sweep, backward stress sweep, backward velocity sweep; each is launched
  * `reps` times back to back between CUDA events on the handle's stream.  The
  * launches overwrite the wavefields of the last run (its records and
- * gradients, already read or accumulated, are untouched). */
+ * gradients, already read or accumulated, are untouched).  The last run must
+ * be a gradient run in the handle's present mode (edge strips, or snapshots
+ * of the same format and interval); SFWI_E_STATE otherwise. */
 int sfwi_time_kernels(sfwi_handle *h, int reps, float *out_ms);
 
 /* Debugging: the packed [X][P] arrays of the batch on the device (X packed

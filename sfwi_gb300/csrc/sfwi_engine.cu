@@ -197,6 +197,9 @@ enum RecArr { R_SYN_Z, R_SYN_X, R_SYN2_Z, R_SYN2_X, R_OBS_Z, R_OBS_X, R_RES_Z, R
 struct Batch {
     int nshots = 0, ntiles = 0, X = 0, P = 0, ntr_tot = 0, max_nxpml = 0;
     bool ready = false;  // the batch described here is the one on the device (its upload completed)
+    // what its run left for gradient steps: snapshots of this mode, or (0) edge strips; neither
+    bool gradient = false;
+    int snap_every = 0, snap_fmt = SNAP_OFF;
     std::vector<ShotGeo> geo;
     std::vector<Tile> tiles;
     std::vector<std::vector<int>> rcols;  // per shot: recording and injection columns (tile flags)
@@ -1175,6 +1178,9 @@ int upload_batch(sfwi_handle *h, const std::vector<ShotIn> &shots, bool forward_
     const size_t recs = (size_t)NREC * std::max(b.ntr_tot, 1) * nt;
     const int nrc = h->stage == 2 ? 4 : 2;
     const bool snap = !forward_only && h->snap_every > 0;
+    b.gradient = !forward_only;
+    b.snap_every = snap ? h->snap_every : 0;
+    b.snap_fmt = snap ? h->snap_fmt : SNAP_OFF;
     b.PS = (b.P + 7) & ~7;
     b.nsnap = snap ? (nt + h->snap_every - 1) / h->snap_every : 0;
     const bool strips = !forward_only && !snap;
@@ -1327,6 +1333,19 @@ int upload_batch(sfwi_handle *h, const std::vector<ShotIn> &shots, bool forward_
     }
     CK(cudaGetLastError());
     return SFWI_OK;
+}
+
+// The batch on the device holds what gradient steps in the handle's present
+// mode read (a Born adjoint's run, or one before sfwi_set_snapshots, left
+// buffers of another mode).
+bool gradient_ready(const sfwi_handle *h) {
+    const Batch &b = h->b;
+    return b.ready && b.gradient && !h->last_forward_only && b.snap_every == h->snap_every &&
+           (b.snap_every == 0 || b.snap_fmt == h->snap_fmt);
+}
+int no_gradient(const sfwi_handle *h) {
+    return fail(SFWI_E_STATE, h->last_forward_only ? "the last run was forward-only (no edge strips)"
+                                                   : "the last run left no gradient state of the present mode");
 }
 
 // The run's stream waits for the observed records issued by upload_batch.
@@ -2643,10 +2662,10 @@ int sfwi_time_kernels(sfwi_handle *h, int reps, float *out_ms) {
     if (!out_ms || reps < 1) return fail(SFWI_E_ARG, "bad argument");
     if (!h->b.ready || h->b.ntiles == 0) return fail(SFWI_E_STATE, "no batch on the device (none run, or the last run failed)");
     CK(cudaSetDevice(h->device));
+    if (!gradient_ready(h)) return no_gradient(h);
     const Params p = make_params(h, false);
     const bool born = h->stage == 2;
     const float adj = h->stage == 1 ? 1.f : -1.f;
-    if (h->last_forward_only) return fail(SFWI_E_STATE, "the last run was forward-only (no edge strips)");
     if (reps > kTimeKernelsMaxReps) reps = kTimeKernelsMaxReps;
     if (reps > h->nt - 1) reps = h->nt - 1;  // step indices 0..reps must exist
     if (reps < 1) return fail(SFWI_E_ARG, "nt too small to time the kernels");
@@ -2678,7 +2697,7 @@ int sfwi_autotune(sfwi_handle *h, int reps, int *choice, float *out_ms) {
     if (int rc = check(h)) return rc;
     if (reps < 1) return fail(SFWI_E_ARG, "bad argument");
     if (!h->b.ready || h->b.ntiles == 0) return fail(SFWI_E_STATE, "no batch on the device (none run, or the last run failed)");
-    if (h->last_forward_only) return fail(SFWI_E_STATE, "the last run was forward-only (no edge strips)");
+    if (!gradient_ready(h)) return no_gradient(h);
     CK(cudaSetDevice(h->device));
     // one gradient step of the batch (the four step kernels) per tile shape;
     // the kernels only read the state and the strips and write the
@@ -2839,7 +2858,7 @@ int sfwi_set_tile_shape(sfwi_handle *h, int shape) {
     build_tiles(h);
     if (int rc = upload_tiles(h)) return rc;
     CK(cudaStreamSynchronize(h->st));  // b.trecs may change again before the copy ran
-    return encode_tile_maps(h, h->last_forward_only);
+    return encode_tile_maps(h, !gradient_ready(h));
 }
 
 int sfwi_get_tile_shape(sfwi_handle *h, int *shape, int *tx, int *tz) {
