@@ -320,10 +320,13 @@ int sfwi_debug_steps(sfwi_handle *h, int *forward, int *backward);
 /* Failure path of the device-side waits, without a fault: runs the tile
  * pipeline of the last batch with a producer that stages nothing and a wait
  * bound of `tries` (1..2^24) mbarrier tries, so the consumers' and the
- * producer's waits run out.  The kernel sets the device error flag and
- * returns, and the call reports it as a run does: SFWI_E_CUDA with "a
- * device-side pipeline wait timed out".  The flag is cleared afterwards and
- * the handle stays usable. */
+ * producer's waits run out.  Where the batch took whole time steps per launch,
+ * one step of each such direction follows, whose waits give up at the first try
+ * and which leaves once its copies have landed (it overwrites the last run's
+ * wavefields).  Each kernel sets the device error flag and returns, and the
+ * call reports it as a run does: SFWI_E_CUDA with "a device-side pipeline wait
+ * timed out" when all of them did.  The flag is cleared afterwards and the
+ * handle stays usable. */
 int sfwi_wait_selftest(sfwi_handle *h, unsigned tries);
 
 /* Source of the forward sweeps.  SFWI_SOURCE_TXX_TZZ (default) is the

@@ -551,8 +551,8 @@ __device__ __forceinline__ void run_tiles(const Params &p, int *counter, Issue i
         if (consumer_any(!ok)) {
             if (threadIdx.x == 0) {
                 atomicExch(p.err, 1);
-                // the other stages may still be loading: let them land (bounded)
-                for (int j = 1; j < NST; j++)
+                // this stage and the others may still be loading: let them land (bounded)
+                for (int j = 0; j < NST; j++)
                     mbar_wait(&full[(k + j) % NST], (uint32_t)(((k + j) / NST) & 1), p.wait_limit);
             }
             return;

@@ -275,6 +275,15 @@ __device__ __forceinline__ Damp2 lane_damp(const float4 &x, const float4 &z, int
                  lane_of<PAIR>(make_float2(z.x, z.z), l), lane_of<PAIR>(make_float2(z.y, z.w), l)};
 }
 
+// A wait ran out: the copies in flight must land before the CTA leaves its
+// shared memory.  Step t waited for full[t & 1]; the copies of step t + 1, if
+// there is one, count on the other.  (PIPE_WAIT_LIMIT whatever the bound of
+// the wait that ran out was)
+__device__ __forceinline__ void drain(uint64_t (&full)[2], int t, int K) {
+    mbar_wait(&full[t & 1], ((t - 2) >> 1) & 1, PIPE_WAIT_LIMIT);
+    if (t + 1 < K) mbar_wait(&full[(t + 1) & 1], ((t - 1) >> 1) & 1, PIPE_WAIT_LIMIT);
+}
+
 struct Item {
     MarchItem m;
     Geo g;
@@ -761,10 +770,9 @@ __global__ void __launch_bounds__((FwdCfg<PS, PAIR, false>::NT), (FwdCfg<PS, PAI
         }
         body.velocity(t - 1);
         if (__syncthreads_or(!ok)) {
-            // a wait ran out: let the copies in flight land (bounded) and leave
             if (tid == 0) {
                 atomicExch(p.err, 1);
-                mbar_wait(&full[(t + 1) & 1], ((t - 1) >> 1) & 1, p.wait_limit);
+                drain(full, t, K);
             }
             return;
         }
@@ -827,7 +835,10 @@ __global__ void __launch_bounds__((FwdCfg<PS, PAIR, true>::NT), 1)
     FwdBody<C, SNAP> body(a, im, sm, it);
     const bool ok = mbar_wait(&full, 0, p.wait_limit);
     if (__syncthreads_or(!ok)) {
-        if (tid == 0) atomicExch(p.err, 1);
+        if (tid == 0) {
+            atomicExch(p.err, 1);
+            mbar_wait(&full, 0, PIPE_WAIT_LIMIT);  // the copies must land before the CTA leaves
+        }
         return;
     }
     if ((im.m.flags & MARCH_SOURCE) && p.src_kind == SRC_TXX_TZZ) {
@@ -1400,10 +1411,9 @@ __global__ void __launch_bounds__((BwdCfg<PS, PAIR, false>::NT), (BwdCfg<PS, PAI
         if (t + 1 < K) next = body.fetch(t + 1);
         body.stress(t - 1);
         if (__syncthreads_or(!ok)) {
-            // a wait ran out: let the copies in flight land (bounded) and leave
             if (tid == 0) {
                 atomicExch(p.err, 1);
-                mbar_wait(&full[(t + 1) & 1], ((t - 1) >> 1) & 1, p.wait_limit);
+                drain(full, t, K);
             }
             return;
         }
@@ -1466,7 +1476,10 @@ __global__ void __launch_bounds__((BwdCfg<PS, PAIR, true>::NT), 1)
     body.fetch_all(K, q);
     const bool ok = mbar_wait(&full, 0, p.wait_limit);
     if (__syncthreads_or(!ok)) {
-        if (tid == 0) atomicExch(p.err, 1);
+        if (tid == 0) {
+            atomicExch(p.err, 1);
+            mbar_wait(&full, 0, PIPE_WAIT_LIMIT);  // the copies must land before the CTA leaves
+        }
         return;
     }
     body.patch_all(q);
