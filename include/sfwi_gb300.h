@@ -310,6 +310,11 @@ int sfwi_debug_grid_shape(sfwi_handle *h, int *X, int *P, int *narrays, int *nst
 int sfwi_debug_tile_grid(int pml, int nzpml, int tx, int tz, const int *nxpml, int nshots, int *z_start,
                          int *x_start, int *tiles, int *frame_tiles);
 int sfwi_debug_read_grid(sfwi_handle *h, int array, float *dst);
+/* Debugging: X*P floats of one of the two copies (0, 1) that the whole steps
+ * of a direction (0 forward, 1 backward) read and write in turn: array 0..9 in
+ * the order of a field's state arrays (the adjoint alone: 0..7), field 1 the
+ * second of a pair.  SFWI_E_STATE where the direction took sweeps. */
+int sfwi_debug_read_copy(sfwi_handle *h, int backward, int copy, int array, int field, float *dst);
 /* Debugging: how the last run's batch took its forward and backward time
  * steps (a forward-only run: backward SFWI_STEPS_SWEEPS). */
 #define SFWI_STEPS_SWEEPS 0 /* a velocity and a stress sweep, one launch each */

@@ -366,6 +366,23 @@ class FD2DGPU_ELASTIC:
             _lib.check(_lib.load().sfwi_debug_read_grid(self._h, a, _fp(out[a])))
         return out, ns.value
 
+    def debug_copies(self):
+        """{(direction, copy, array, field): [X, P] float32} of the copies of
+        the fields that the last run's whole steps advanced."""
+        X, P, na, ns = C.c_int(), C.c_int(), C.c_int(), C.c_int()
+        _lib.check(_lib.load().sfwi_debug_grid_shape(self._h, C.byref(X), C.byref(P), C.byref(na), C.byref(ns)))
+        out = {}
+        for back, way in enumerate(self.debug_steps()):
+            if way == "sweeps":
+                continue
+            single = self.stage == 1 if not back else getattr(self, "_snap", None) is not None
+            for copy in range(2):
+                for array in range(8 if back and single else 10):
+                    for field in range(1 if single else 2):
+                        a = out[back, copy, array, field] = np.zeros((X.value, P.value), np.float32)
+                        _lib.check(_lib.load().sfwi_debug_read_copy(self._h, back, copy, array, field, _fp(a)))
+        return out
+
     def debug_steps(self):
         """How the last run's batch took its (forward, backward) time steps:
         "sweeps", or whole steps per launch as a "march" or a "burst"."""

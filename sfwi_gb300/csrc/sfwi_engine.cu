@@ -1026,6 +1026,30 @@ void start_backward(sfwi_handle *h) {
     launch_pair_start(s, b.max_nxpml, b.nshots, h->st);
     h->launches++;
 }
+// Where a shot's array of `grid`'s state, as the sweeps would leave it, lies
+// after whole steps (layout_march): its first element and the distance of
+// neighbouring cells; null: zeros.  A shot's forward steps end in a copy that
+// its own length decides; backward steps end in the first.
+struct FieldAt {
+    const float *p;
+    size_t stride;
+};
+FieldAt field_at(const sfwi_handle *h, int array, int shot) {
+    const Batch &b = h->b;
+    const int nt = b.aux[shot].nt, last = (b.gradient ? nt : nt + h->nt) & 1;
+    const FieldAt grid{b.grid.p + (size_t)array * b.cells, 1};
+    auto pair = [&](const float *copy, int k, int field) { return FieldAt{copy + 2 * k * b.cells + field, 2}; };
+    if (array >= AD_VX)  // the adjoint
+        return b.bwd_pairs ? pair(b.bwd_copy[0], array == AD_MTXZ ? BG_MTXZ : array - AD_VX, 1) : grid;
+    if (array >= SC_VX) {  // the scattered field: the forward steps' last, unless the adjoint took its place
+        if (h->stage == 1 || (b.way[0] && b.bwd_pairs)) return FieldAt{nullptr, 0};
+        return b.way[0] ? pair(b.fwd_copy[last], array - SC_VX, 1) : grid;
+    }
+    // the reconstruction; in snapshot and forward-only runs the background
+    if (b.gradient && b.snap_every == 0) return b.bwd_pairs ? pair(b.bwd_copy[0], array, 0) : grid;
+    if (!b.way[0]) return grid;
+    return b.fwd_pairs ? pair(b.fwd_copy[last], array, 0) : FieldAt{b.fwd_copy[last] + array * b.cells, 1};
+}
 int march_count(const Batch &b, int it, bool backward) {
     const std::vector<int> &act = b.items_active[backward];
     return act.empty() ? (int)b.items[backward].size() : act[it];
@@ -2757,36 +2781,40 @@ int sfwi_debug_read_grid(sfwi_handle *h, int array, float *dst) {
     Batch &b = h->b;
     if (!b.ready) return fail(SFWI_E_STATE, "no batch on the device");
     CK(cudaSetDevice(h->device));
-    // after whole steps per launch the fields lie in their own layout
-    // (layout_march); the last step wrote the first copy.  The backward steps
-    // keep no scattered field.
     if ((b.way[0] || b.way[1]) && array < G_LAM) {
-        const bool back = !h->last_forward_only;
-        if (array >= SC_VX && array < AD_VX && back && h->stage == 2 && b.bwd_pairs) {
-            std::memset(dst, 0, b.cells * sizeof(float));
-            return SFWI_OK;
+        if (!b.grid2.p) return fail(SFWI_E_STATE, "the last run's copies of the fields were given back");
+        for (int k = 0; k < b.nshots; k++) {
+            const ShotGeo &g = b.geo[k];
+            const size_t off = (size_t)g.row0 * b.P, n = (size_t)g.nxpml * b.P;
+            const FieldAt f = field_at(h, array, k);
+            if (f.p)
+                CK(cudaMemcpy2DAsync(dst + off, sizeof(float), f.p + off * f.stride, f.stride * sizeof(float),
+                                     sizeof(float), n, cudaMemcpyDeviceToHost, h->st));
+            else
+                std::memset(dst + off, 0, n * sizeof(float));
         }
-        const float *src = nullptr;
-        size_t stride = 2;
-        const int copy = back ? h->nt & 1 : 0;  // where the forward steps ended
-        if (back && b.bwd_pairs && (array < SC_VX || array >= AD_VX)) {
-            // reconstruction, adjoint
-            const int k = array < SC_VX ? array : array == AD_MTXZ ? BG_MTXZ : array - AD_VX;
-            src = b.bwd_copy[0] + 2 * (size_t)k * b.cells + (array >= AD_VX);
-        } else if (b.fwd_pairs && array < AD_VX && !(back && array < SC_VX && h->snap_every == 0)) {
-            src = b.fwd_copy[copy] + 2 * (size_t)(array % SC_VX) * b.cells + (array >= SC_VX);
-        } else if (b.way[0] && array < SC_VX && h->snap_every > 0) {
-            src = b.fwd_copy[copy] + (size_t)array * b.cells;
-            stride = 1;
-        }
-        if (src) {
-            CK(cudaMemcpy2DAsync(dst, sizeof(float), src, stride * sizeof(float), sizeof(float), b.cells,
-                                 cudaMemcpyDeviceToHost, h->st));
-            CK(cudaStreamSynchronize(h->st));
-            return SFWI_OK;
-        }
+        CK(cudaStreamSynchronize(h->st));
+        return SFWI_OK;
     }
     CK(cudaMemcpyAsync(dst, b.g(array), b.cells * sizeof(float), cudaMemcpyDeviceToHost, h->st));
+    CK(cudaStreamSynchronize(h->st));
+    return SFWI_OK;
+}
+
+int sfwi_debug_read_copy(sfwi_handle *h, int backward, int copy, int array, int field, float *dst) {
+    if (int rc = check(h)) return rc;
+    Batch &b = h->b;
+    if (!b.ready || !b.way[backward != 0] || !b.grid2.p)
+        return fail(SFWI_E_STATE, "no copies of the fields: the steps were sweeps");
+    const bool pairs = backward ? b.bwd_pairs : b.fwd_pairs;
+    if (!dst || copy < 0 || copy > 1 || array < 0 || array >= (backward && !pairs ? 8 : 10) || field < 0 ||
+        field > (pairs ? 1 : 0))
+        return fail(SFWI_E_ARG, "bad copy %d, array %d, field %d", copy, array, field);
+    CK(cudaSetDevice(h->device));
+    const size_t stride = pairs ? 2 : 1;
+    const float *src = (backward ? b.bwd_copy : b.fwd_copy)[copy] + stride * array * b.cells + field;
+    CK(cudaMemcpy2DAsync(dst, sizeof(float), src, stride * sizeof(float), sizeof(float), b.cells,
+                         cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));
     return SFWI_OK;
 }
