@@ -315,6 +315,9 @@ int sfwi_debug_read_grid(sfwi_handle *h, int array, float *dst);
  * the order of a field's state arrays (the adjoint alone: 0..7), field 1 the
  * second of a pair.  SFWI_E_STATE where the direction took sweeps. */
 int sfwi_debug_read_copy(sfwi_handle *h, int backward, int copy, int array, int field, float *dst);
+/* Debugging: allocations that take the handle's device buffers beyond `bytes`
+ * fail as on a full device (SFWI_E_NOMEM); *used (optional) gets what they hold. */
+int sfwi_debug_memory_limit(sfwi_handle *h, size_t bytes, size_t *used);
 /* Debugging: how the last run's batch took its forward and backward time
  * steps (a forward-only run: backward SFWI_STEPS_SWEEPS). */
 #define SFWI_STEPS_SWEEPS 0 /* a velocity and a stress sweep, one launch each */

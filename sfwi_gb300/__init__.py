@@ -383,6 +383,14 @@ class FD2DGPU_ELASTIC:
                         _lib.check(_lib.load().sfwi_debug_read_copy(self._h, back, copy, array, field, _fp(a)))
         return out
 
+    def debug_memory_limit(self, nbytes=None):
+        """Have allocations beyond `nbytes` of device memory fail (None: no
+        limit); returns the bytes that the engine's buffers hold."""
+        used = C.c_size_t()
+        _lib.check(_lib.load().sfwi_debug_memory_limit(self._h, C.c_size_t(-1).value if nbytes is None else int(nbytes),
+                                                       C.byref(used)))
+        return used.value
+
     def debug_steps(self):
         """How the last run's batch took its (forward, backward) time steps:
         "sweeps", or whole steps per launch as a "march" or a "burst"."""

@@ -53,26 +53,31 @@ int fail(int code, const char *fmt, ...) {
                         #call, cudaGetErrorString(e_), __FILE__, __LINE__);                             \
     } while (0)
 
+// bytes in the device buffers of a handle, and their limit (sfwi_debug_memory_limit)
+struct MemUse {
+    size_t used = 0, limit = SIZE_MAX;
+};
+
 // Device buffer that grows on demand.  With a stream attached, allocation
 // and release are stream-ordered (cudaMallocAsync / cudaFreeAsync on the
 // owning handle's stream), so a handle that grows or frees its buffers never
-// waits for work other handles have in flight on the same device.
+// waits for work other handles have in flight on the same device.  A buffer
+// that finds no memory has the handle's spare one given back and tries again.
 template <class T>
 struct DevBuf {
     T *p = nullptr;
     size_t n = 0;
     cudaStream_t st = nullptr;
+    MemUse *mem = nullptr;
+    DevBuf<float> *spare = nullptr;
     cudaError_t ensure(size_t m) {
         if (m <= n && p) return cudaSuccess;
         release();
-        const size_t bytes = std::max<size_t>(m, 1) * sizeof(T);
-        cudaError_t e = st ? cudaMallocAsync(reinterpret_cast<void **>(&p), bytes, st)
-                           : cudaMalloc(reinterpret_cast<void **>(&p), bytes);
-        if (e == cudaSuccess) {
-            n = m;
-        } else {
-            p = nullptr;
-            cudaGetLastError();  // the failure is returned here; later launch checks must not see it again
+        cudaError_t e = alloc(m);
+        if (e == cudaErrorMemoryAllocation && spare && spare->p && static_cast<void *>(spare) != this) {
+            spare->release();
+            cudaStreamSynchronize(st);
+            e = alloc(m);
         }
         return e;
     }
@@ -82,9 +87,27 @@ struct DevBuf {
                 cudaFreeAsync(p, st);
             else
                 cudaFree(p);
+            if (mem) mem->used -= bytes(n);
         }
         p = nullptr;
         n = 0;
+    }
+
+private:
+    static size_t bytes(size_t m) { return std::max<size_t>(m, 1) * sizeof(T); }
+    cudaError_t alloc(size_t m) {
+        const size_t b = bytes(m);
+        if (mem && (mem->used > mem->limit || b > mem->limit - mem->used)) return cudaErrorMemoryAllocation;
+        cudaError_t e = st ? cudaMallocAsync(reinterpret_cast<void **>(&p), b, st)
+                           : cudaMalloc(reinterpret_cast<void **>(&p), b);
+        if (e == cudaSuccess) {
+            n = m;
+            if (mem) mem->used += b;
+        } else {
+            p = nullptr;
+            cudaGetLastError();  // the failure is returned here; later launch checks must not see it again
+        }
+        return e;
     }
 };
 
@@ -240,7 +263,7 @@ struct Batch {
     // they take (null: the sweeps), the second copy of the fields, the items,
     // tensor maps reading either copy
     const MarchVariant *way[2] = {nullptr, nullptr};
-    DevBuf<float> grid2;     // further copies of the fields, and the PML factors
+    DevBuf<float> grid2;     // further copies of the fields, and the PML factors: the handle's spare buffer
     float *fwd_copy[2] = {nullptr, nullptr}, *bwd_copy[2] = {nullptr, nullptr};
     bool fwd_pairs = false, bwd_pairs = false;  // two fields as float2 per cell
     float *fx = nullptr, *fz = nullptr;  // PML factors
@@ -284,6 +307,7 @@ struct sfwi_handle {
     int isx = 0, isz = 0, igz = 0, ngx_left = 0, delta_left = 0, record_left_in_v = 0;
     bool have_geom = false, have_rec = false;
     std::vector<ShotIn> queue;
+    MemUse mem;
     Batch b;
     std::vector<int> last_ntr;   // traces of each shot of the last run
     std::vector<int> last_tr0;
@@ -928,16 +952,19 @@ void plan_march(sfwi_handle *h, bool forward_only) {
 
 // The second copy of the fields, the item tables and the tensor maps.  The
 // copy is taken only where memory is plentiful (an eighth of what is free): the run
-// takes the sweeps otherwise, which need none.
+// takes the sweeps otherwise, which need none.  It comes after every other
+// buffer of the run, and is given back when a later run's buffer finds no memory.
 int upload_march(sfwi_handle *h, bool forward_only) {
     Batch &b = h->b;
     if (!b.way[0] && !b.way[1]) return SFWI_OK;
-    const size_t n = layout_march(h, forward_only);
-    bool have = n <= b.grid2.n && b.grid2.p;
-    if (!have) {
+    const size_t n = layout_march(h, forward_only), nf = b.items[0].size(), nb = b.items[1].size();
+    // (the items first: they may have an earlier run's copy given back)
+    bool have = b.ditems.ensure(nf + nb) == cudaSuccess;
+    if (have && !(n <= b.grid2.n && b.grid2.p)) {
         size_t free_bytes = 0, total = 0;
         b.grid2.release();
         CK(cudaMemGetInfo(&free_bytes, &total));
+        free_bytes = std::min(free_bytes, h->mem.limit - std::min(h->mem.used, h->mem.limit));
         have = n * sizeof(float) <= free_bytes / 8 && b.grid2.ensure(n) == cudaSuccess;
     }
     if (!have) {
@@ -946,8 +973,6 @@ int upload_march(sfwi_handle *h, bool forward_only) {
     }
     layout_march(h, forward_only);  // now with the buffer in place
     CK(cudaMemsetAsync(b.grid2.p, 0, n * sizeof(float), h->st));
-    const size_t nf = b.items[0].size(), nb = b.items[1].size();
-    CK(b.ditems.ensure(nf + nb));
     if (nf) CK(cudaMemcpyAsync(b.ditems.p, b.items[0].data(), nf * sizeof(MarchItem), cudaMemcpyHostToDevice, h->st));
     if (nb)
         CK(cudaMemcpyAsync(b.ditems.p + nf, b.items[1].data(), nb * sizeof(MarchItem), cudaMemcpyHostToDevice, h->st));
@@ -1264,6 +1289,8 @@ int upload_batch(sfwi_handle *h, const std::vector<ShotIn> &shots, bool forward_
     CK(b.drtr.ensure(b.rtr.size()));
     CK(b.daux.ensure(b.aux.size()));
     if (!b.tlen.empty()) CK(b.dtlen.ensure(b.tlen.size()));
+    if (with_obs && !h->force_l2 && h->misfit_kind != SFWI_MISFIT_L2)
+        if (const size_t nscr = ot_scratch_doubles(nt, b.ntr_tot)) CK(b.otscr.ensure(nscr));
     CK(b.derr.ensure(1));
     CK(cudaMemsetAsync(b.derr.p, 0, sizeof(int), h->st));
     const size_t nctr = 4 * (size_t)std::max(h->nt, kTimeKernelsMaxReps + 1);
@@ -1603,13 +1630,6 @@ int run_batch(sfwi_handle *h, const std::vector<ShotIn> &shots, int mode, double
     ObservedGuard obs_guard{h};
     plan_march(h, forward_only);
     rc = upload_batch(h, shots, forward_only, mode != RUN_FORWARD);
-    if (rc == SFWI_E_NOMEM && h->b.grid2.p) {
-        // an earlier run's copy of the fields may hold what this one needs
-        CK(cudaStreamSynchronize(h->st));
-        h->b.grid2.release();
-        no_march(h->b);
-        rc = upload_batch(h, shots, forward_only, mode != RUN_FORWARD);
-    }
     if (rc) return rc;
     Batch &b = h->b;
     b.ready = true;
@@ -1688,10 +1708,7 @@ int run_batch(sfwi_handle *h, const std::vector<ShotIn> &shots, int mode, double
         o.res_x = b.r(R_RES_X, nt);
         o.sigma = b.dsigma.p;
         o.trace_misfit = b.tmis.p;
-        if (const size_t nscr = ot_scratch_doubles(nt, b.ntr_tot)) {
-            CK(b.otscr.ensure(nscr));
-            o.scratch = b.otscr.p;
-        }
+        if (ot_scratch_doubles(nt, b.ntr_tot)) o.scratch = b.otscr.p;
         CK(launch_ot(o, st));
     }
     if (mode == RUN_MISFIT) return finish_misfit(h, misfit_kind, misfit, per_shot);
@@ -2213,7 +2230,7 @@ int sfwi_create(sfwi_handle **out, int stage, const float *sou, float dx, float 
             rc = fail(SFWI_E_CUDA, "stream: %s", cudaGetErrorString(e));
             break;
         }
-        for_each_buf(h, [h](auto &d) { d.st = h->st; });
+        for_each_buf(h, [h](auto &d) { d.st = h->st, d.mem = &h->mem, d.spare = &h->b.grid2; });
         for (auto &ev : h->ev)
             if ((e = cudaEventCreate(&ev)) != cudaSuccess) {
                 rc = fail(SFWI_E_CUDA, "event: %s", cudaGetErrorString(e));
@@ -2816,6 +2833,13 @@ int sfwi_debug_read_copy(sfwi_handle *h, int backward, int copy, int array, int 
     CK(cudaMemcpy2DAsync(dst, sizeof(float), src, stride * sizeof(float), sizeof(float), b.cells,
                          cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));
+    return SFWI_OK;
+}
+
+int sfwi_debug_memory_limit(sfwi_handle *h, size_t bytes, size_t *used) {
+    if (int rc = check(h)) return rc;
+    h->mem.limit = bytes;
+    if (used) *used = h->mem.used;
     return SFWI_OK;
 }
 
