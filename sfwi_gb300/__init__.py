@@ -414,6 +414,13 @@ class FD2DGPU_ELASTIC:
         """Programmatic dependent launch of the time-step kernels (default on)."""
         _lib.check(_lib.load().sfwi_set_launch_overlap(self._h, int(bool(on))))
 
+    def set_copy_limit(self, nbytes=None):
+        """Bytes that the copies of the wavefields of whole time steps may take
+        in later runs (None: an eighth of the free device memory, the
+        default, which holds beside any limit); runs that would need more take
+        the sweeps.  Results do not depend on it."""
+        _lib.check(_lib.load().sfwi_set_copy_limit(self._h, C.c_size_t(-1).value if nbytes is None else int(nbytes)))
+
     def set_tile_order(self, reverse_bits):
         """Bit k: time-step sweep k (forward velocity, forward stress,
         backward stress, backward velocity) draws its tiles in reverse table

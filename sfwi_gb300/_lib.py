@@ -77,6 +77,7 @@ SIGNATURES = {
     "sfwi_debug_read_grid": (C.c_int, [_h, C.c_int, _fp]),
     "sfwi_debug_read_copy": (C.c_int, [_h, C.c_int, C.c_int, C.c_int, C.c_int, _fp]),
     "sfwi_debug_memory_limit": (C.c_int, [_h, C.c_size_t, C.POINTER(C.c_size_t)]),
+    "sfwi_set_copy_limit": (C.c_int, [_h, C.c_size_t]),
     "sfwi_debug_steps": (C.c_int, [_h, _ip, _ip]),
     "sfwi_debug_tile_grid": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, _ip, C.c_int, C.POINTER(C.c_int), _ip,
                                        _ip, _ip]),

@@ -321,6 +321,7 @@ struct sfwi_handle {
     const TileVariant *tv = nullptr;  // tile shape of the step kernels
     bool tile_auto = true;            // shape picked per batch by its size (until one is set)
     bool march_ok = true;             // large enough batches may run whole steps per launch
+    size_t copy_limit = SIZE_MAX;     // bytes that their copies of the fields may take
     int nsm = 0;                      // multiprocessors of the device
     // trial models of a line search: while set, shots cut their windows from
     // these slot arrays instead of the uploaded model
@@ -956,6 +957,7 @@ void plan_march(sfwi_handle *h, bool forward_only) {
 // buffer of the run, and is given back when a later run's buffer finds no memory.
 int upload_march(sfwi_handle *h, bool forward_only) {
     Batch &b = h->b;
+    if (b.grid2.n * sizeof(float) > h->copy_limit) b.grid2.release();
     if (!b.way[0] && !b.way[1]) return SFWI_OK;
     const size_t n = layout_march(h, forward_only), nf = b.items[0].size(), nb = b.items[1].size();
     // (the items first: they may have an earlier run's copy given back)
@@ -965,7 +967,7 @@ int upload_march(sfwi_handle *h, bool forward_only) {
         b.grid2.release();
         CK(cudaMemGetInfo(&free_bytes, &total));
         free_bytes = std::min(free_bytes, h->mem.limit - std::min(h->mem.used, h->mem.limit));
-        have = n * sizeof(float) <= free_bytes / 8 && b.grid2.ensure(n) == cudaSuccess;
+        have = n * sizeof(float) <= std::min(free_bytes / 8, h->copy_limit) && b.grid2.ensure(n) == cudaSuccess;
     }
     if (!have) {
         no_march(b);
@@ -2904,6 +2906,12 @@ int sfwi_set_source(sfwi_handle *h, int kind) {
 int sfwi_set_launch_overlap(sfwi_handle *h, int on) {
     if (int rc = check(h)) return rc;
     h->launch_overlap = on != 0;
+    return SFWI_OK;
+}
+
+int sfwi_set_copy_limit(sfwi_handle *h, size_t bytes) {
+    if (int rc = check(h)) return rc;
+    h->copy_limit = bytes;
     return SFWI_OK;
 }
 

@@ -82,8 +82,7 @@ def request_bytes(req, strip_chunk=0):
     """Device memory of one request's engine (the engine's allocations,
     sfwi_engine.cu:upload_batch, plus the model and the FP64 gradients);
     strip_chunk > 0: edge strips in host memory in chunks of that many steps.
-    The engine's optional second copy of the wavefields is not counted: it is
-    taken only from memory that is plentiful."""
+    The engine's optional copies of the wavefields come on top (copy_bytes)."""
     P = (req.allnz + 2 * req.pml + 3) // 4 * 4
     X = sum(int(d["nx"]) + 2 * req.pml for d in req.shots)
     ntr = sum(len(d["gc"]) for d in req.shots)
@@ -115,9 +114,19 @@ def batch_bytes(reqs, strip_chunk=0):
     return 4 * floats + 8 * 4 * cells + (1 << 20)
 
 
-def run_requests(reqs, strip_chunk=0):
+def copy_bytes(reqs):
+    """The most that the copies of the wavefields of whole time steps take in
+    one run of the requests: 44 arrays of the packed grid (layout_march,
+    sfwi_engine.cu, stage 1)."""
+    pml = reqs[0].pml
+    P = (max(r.allnz for r in reqs) + 2 * pml + 3) // 4 * 4
+    return 4 * 44 * P * sum(int(d["nx"]) + 2 * pml for r in reqs for d in r.shots)
+
+
+def run_requests(reqs, strip_chunk=0, copy_limit=None):
     """Several requests in one run of one engine (sfwi_run_models): a list of
-    (misfit, grad_pp, grad_ps, illum), one per request."""
+    (misfit, grad_pp, grad_ps, illum), one per request.  copy_limit: see
+    set_copy_limit."""
     import sfwi_gb300 as sg
     pml, dx, dt = reqs[0].pml, reqs[0].dx, reqs[0].dt
     for r in reqs:
@@ -138,6 +147,7 @@ def run_requests(reqs, strip_chunk=0):
             fd.set_misfit(reqs[0].misfit_kind)
         if strip_chunk:
             fd.set_cpu_mem(1, strip_chunk)
+        fd.set_copy_limit(copy_limit)
         shot_model = []
         for k, r in enumerate(reqs):
             for d in r.shots:
@@ -165,7 +175,7 @@ def request_work(req):
     return sum((int(d["nx"]) + 2 * req.pml) * P for d in req.shots) * req.nt
 
 
-def run_request(req, strip_chunk=0):
+def run_request(req, strip_chunk=0, copy_limit=None):
     """One request on a fresh engine: (misfit, grad_pp, grad_ps, illum)."""
     import sfwi_gb300 as sg
     maxnx = max(int(d["nx"]) for d in req.shots)
@@ -177,6 +187,7 @@ def run_request(req, strip_chunk=0):
             fd.set_misfit(req.misfit_kind)
         if strip_chunk:
             fd.set_cpu_mem(1, strip_chunk)
+        fd.set_copy_limit(copy_limit)
         for d in req.shots:
             fd.enqueue_shot(d["nx"], d["isx"], d["isz"], d["igz"], d["ngx_left"], d["delta_left"], 0, d["gc"],
                             d["obs_z"], d["obs_x"])
@@ -200,7 +211,10 @@ class Server:
     Batched (batch=True): the requests admitted together share one run, at
     most max_batch of them.  strip_chunk > 0 keeps every run's edge strips in host memory
     in chunks of that many steps (sfwi_set_cpu_mem): the budget then counts
-    the device ring only, and more requests fit at once.  During run() the
+    the device ring only, and more requests fit at once.  A run may take copies
+    of the wavefields for whole time steps where they fit in an eighth of what
+    it leaves of the budget, which counts them while it runs (a runner of
+    the caller's own is given no copies to count).  During run() the
     pinned blocks that finished engines release are kept (up to
     pinned_cache_bytes) for the next engines, and freed when it returns."""
 
@@ -212,13 +226,14 @@ class Server:
         self.budget = int(budget_bytes)
         self.max_active = int(max_active)
         sc = int(strip_chunk)
-        self.runner = runner or (lambda r: run_request(r, sc))
+        self.own_runner = (batch_runner if batch else runner) is None
+        self.runner = runner or (lambda r, copy=None: run_request(r, sc, copy))
         self.sizer = sizer or (lambda r: request_bytes(r, sc))
         self.clock = clock
         self.policy, self.work = policy, work
         # batched: the requests admitted together share one run (batch_runner)
         self.batch = batch
-        self.batch_runner = batch_runner or (lambda g: run_requests(g, sc))
+        self.batch_runner = batch_runner or (lambda g, copy=None: run_requests(g, sc, copy))
         self.batch_sizer = batch_sizer or (lambda g: batch_bytes(g, sc))
         self.max_batch = int(max_batch)
         self.window = float(window)
@@ -251,9 +266,15 @@ class Server:
         def now():
             return self.clock() - t0
 
-        def worker(group, size, admitted):
+        def copies(group, left):
+            # what the group's run may take beside its own size, of `left` bytes
+            need = copy_bytes(group) if self.own_runner else 0
+            return need if 8 * need <= left else 0
+
+        def worker(group, size, admitted, copy):
+            arg = (copy,) if self.own_runner else ()
             try:
-                outs = self.batch_runner(group) if self.batch else [self.runner(group[0])]
+                outs = self.batch_runner(group, *arg) if self.batch else [self.runner(group[0], *arg)]
                 done = now()
                 with cv:
                     for r, out in zip(group, outs):
@@ -263,7 +284,7 @@ class Server:
                     errors.append(e)
             finally:
                 with cv:
-                    state["used"] -= size
+                    state["used"] -= size + copy
                     state["active"] -= 1
                     cv.notify_all()
 
@@ -295,9 +316,10 @@ class Server:
                         if group:
                             for r in group:
                                 waiting.remove(r)
-                            state["used"] += size
+                            copy = copies(group, self.budget - state["used"] - size)
+                            state["used"] += size + copy
                             state["active"] += 1
-                            th = threading.Thread(target=worker, args=(group, size, now()), daemon=True)
+                            th = threading.Thread(target=worker, args=(group, size, now(), copy), daemon=True)
                             th.start()
                             threads.append(th)
                     order = []
@@ -307,9 +329,10 @@ class Server:
                     size = self.sizer(r)
                     if state["used"] + size <= self.budget:
                         waiting.remove(r)
-                        state["used"] += size
+                        copy = copies([r], self.budget - state["used"] - size)
+                        state["used"] += size + copy
                         state["active"] += 1
-                        th = threading.Thread(target=worker, args=([r], size, now()), daemon=True)
+                        th = threading.Thread(target=worker, args=([r], size, now(), copy), daemon=True)
                         th.start()
                         threads.append(th)
                     elif self.max_active == 1:
