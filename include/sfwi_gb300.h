@@ -269,9 +269,9 @@ int sfwi_ot_alltrace(const float *obs_x, const float *obs_z, const float *cal_x,
  * calls fail with SFWI_E_ARG before any device work) and length <= 7160.
  * The first call in a CUDA context looks up that array's device address
  * (cudaGetSymbolAddress), so make it before any stream capture.  All calls
- * on a device share the array and each call overwrites what the last one
- * left there: calls that overlap on the GPU (other streams or threads at the
- * same time) race on it and must be serialised by the caller. */
+ * on a device share the array: calls of several threads, on whatever streams,
+ * take turns (each holds the device's lock until its work has ended).
+ * Processes have an array each. */
 int sfwi_ot_noalloc(int kind, const float *obs_x, const float *obs_z, const float *cal_x, const float *cal_z,
                     float *res_x, float *res_z, int length, int tracenum, float dt, double *misfit, void *stream);
 /* normalize(matrix, length, tracenum), sfwi-stage1/main.cpp:24-32: divide by

@@ -668,8 +668,9 @@ cudaError_t launch_ot_gather(const OtArgs &a, cudaStream_t st) {
 // up front, and inner loops where a cudaMalloc/cudaFree may synchronise the
 // device and stall other work in flight.
 // Every device that loads this library holds the array (256 KB) until the
-// process exits.  All calls on a device share it, so calls that overlap on the
-// GPU (different streams or threads at the same time) race on it.
+// process exits.  All calls on a device share it: a call holds the device's lock
+// from its first launch until its work has ended, so calls from several
+// threads, on whatever streams, take turns.
 // ---------------------------------------------------------------------------
 constexpr int OT_NOALLOC_MAX_TRACES = 8192;
 // [0, 2*max): scale per (trace, component); [2*max, 4*max): misfit per
@@ -759,7 +760,8 @@ struct ScratchAddr {
     unsigned long long ctx;
     double *addr;
 };
-std::mutex g_noalloc_mu;
+std::mutex g_noalloc_mu;            // of the addresses
+std::mutex g_noalloc_call[128];     // of each device's array
 ScratchAddr g_noalloc_addr[128] = {};
 
 unsigned long long current_context_id() {
@@ -826,6 +828,7 @@ extern "C" int sfwi_ot_noalloc(int kind, const float *obs_x, const float *obs_z,
     }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     double *sigma = scratch, *tmis = scratch + 2 * OT_NOALLOC_MAX_TRACES, *sum = scratch + 4 * OT_NOALLOC_MAX_TRACES;
+    std::lock_guard<std::mutex> turn(g_noalloc_call[dev]);
     k_ot_trace_scale<<<2 * tracenum, 256, 0, st>>>(obs_z, obs_x, length, sigma);
     k_ot_gather_scale<<<2, 256, 0, st>>>(sigma, tracenum, kind == 3);
     OtArgs o{};
@@ -842,12 +845,14 @@ extern "C" int sfwi_ot_noalloc(int kind, const float *obs_x, const float *obs_z,
     o.res_x = res_x;
     o.sigma = sigma;
     o.trace_misfit = tmis;
-    if ((e = launch_ot_gather(o, st)) != cudaSuccess) return record_error(-2, "sfwi_ot_noalloc: %s", cudaGetErrorString(e));
-    k_ot_sum<<<1, 1024, 0, st>>>(tmis, tracenum, sum);
     double w = 0.0;
-    if ((e = cudaMemcpyAsync(&w, sum, sizeof(double), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(st)) != cudaSuccess)
-        return record_error(-2, "sfwi_ot_noalloc: %s", cudaGetErrorString(e));
+    if ((e = launch_ot_gather(o, st)) == cudaSuccess) {
+        k_ot_sum<<<1, 1024, 0, st>>>(tmis, tracenum, sum);
+        e = cudaMemcpyAsync(&w, sum, sizeof(double), cudaMemcpyDeviceToHost, st);
+    }
+    const cudaError_t end = cudaStreamSynchronize(st);  // (also after an error: the array is the next call's)
+    if (e == cudaSuccess) e = end;
+    if (e != cudaSuccess) return record_error(-2, "sfwi_ot_noalloc: %s", cudaGetErrorString(e));
     *misfit += w;
     return 0;
 }
