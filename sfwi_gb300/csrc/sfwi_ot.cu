@@ -517,7 +517,7 @@ __global__ void __maxnreg__(56) k_ot(OtArgs a, int run) {
 
     // weights, the sums of both runs, and the CDF G of the observed trace
     u64 F = 0, offG = 0;
-    bool bad = false;
+    bool bad = POWER && inv_sigma == 0.0;  // (an infinite sigma, and with it every weight)
     for (int k = k0; k < k1; k++) {
         const D2 x = weight(U[k], mc, ec), y = weight(O[k], mo, eo);
         bad |= !(x.h <= 2.f && y.h <= 2.f);
