@@ -27,20 +27,26 @@
 // the other's after 3000 steps (as far as each is from FP64), so gradient
 // runs stay with the FP64 form and their bits.
 // The integers: CDFs are sums of positive weights, in units of 2^-s of the
-// largest one, s such that a trace's sum stays below 2^62.  Integer sums are
+// largest one, s such that a trace's sum stays below 2^62 (OT_power's weights are
+// integers from the start, from the exact square of u's 24 bits).  Integer sums are
 // exact in any order, so F_k - G_{m-1} and the search have no rounding but the weights'
-// own (2^-50 at 3000 samples), and equal traces have equal CDFs.  What
-// follows the search (r, its square, the adjoint weights and their sums) is in
-// float pairs of 48 bits (D2, sfwi_d2.cuh); its cancellation of nearly equal numbers,
-// k+1 - T_k, is done in integers before.  Against FP64 the errors are those of the FP64
-// kernel: residuals the same to six digits, misfits at 1e-14.
-// In both the exponential weights are FP32 (expf of the argument rounded to FP32):
-// their argument is at most 0, so a weight is 1 at the trace's maximum and
-// its relative rounding of about 1e-7 stays far below the 1e-4 parity bar.
+// own (2^-50 at 3000 samples) and that of the ratio of the sums, 2^-63, upwards:
+// densities of equal shape have equal CDFs.  What follows the search (r, its
+// square, the adjoint weights and their sums) is in float pairs of 48 bits
+// (D2, sfwi_d2.cuh).  The two cancellations are kept out of them: k+1 - T_k
+// is done in integers, and A_j - sum f A relative to A at the largest weight,
+// which matters where one sample holds nearly all of it.
+// In both kernels the exponential weights are FP32 (expf of the argument rounded to
+// FP32): their argument is at most 0, so a weight is 1 at the trace's maximum and
+// its relative rounding of about 1e-7 stays far below the 1e-4 parity bar.  Against the
+// formulas in quad precision, over 3000 random gathers: residuals (median) 2.9e-7 and
+// misfits 9e-9 for OT, 1.8e-7 and 2e-8 for OT_alltrace in either kernel, from those
+// weights; OT_power residuals 2.6e-8 in either, misfits 1.5e-15 (k_ot_fp64 4e-16).
 // One CTA handles one (trace, component); prefix and suffix sums are block
 // scans built on warp shuffles.
 #include <algorithm>
 #include <cfloat>
+#include <climits>
 #include <cudaTypedefs.h>
 #include <mutex>
 
@@ -404,10 +410,10 @@ __global__ void __maxnreg__(56) k_ot(OtArgs a, int run) {
     // per-trace constants, formed by thread 0 in FP64
     __shared__ struct {
         float mc, mo;
-        double inv_sigma, scale;
-        D2 is, c, norm, sc, FA;
-        u64 ratio;
-        int wide, ec, eo, bc, bo, shift;
+        double inv_sigma, inv_S, scale;  // inv_S: of p's units
+        D2 is, c, norm, sc, ref, FA;
+        u64 ratio, kc, ko, least_c, least_o;
+        int wide, ec, eo, bc, bo, shift, sc2, so2, kref;
     } tc;
     const int n = a.nt;
     // G: CDF of the observed trace; B: the adjoint weights but for a constant
@@ -453,7 +459,8 @@ __global__ void __maxnreg__(56) k_ot(OtArgs a, int run) {
         double sigma = a.sigma[2 * tr + comp];
         if (!(sigma > 0.0)) sigma = 1.0;
         const double inv = 1.0 / sigma;
-        tc.mc = mc, tc.mo = mo;
+        tc.mc = POWER ? ac : mc, tc.mo = mo;
+        tc.kref = INT_MAX, tc.ref = D2{0.f, 0.f};
         tc.inv_sigma = inv;
         tc.is = to_d2(inv);
         // Scales at which a float pair could overflow or lose bits: the
@@ -486,32 +493,39 @@ __global__ void __maxnreg__(56) k_ot(OtArgs a, int run) {
         if (threadIdx.x == 0) {
             // (a margin for the rounding of these sums)
             auto room = [&](float t) {
-                return t > 0.f ? min(max(all_ones, 62 - (ilogbf(1.01f * t) + 1)), 62) : all_ones;
+                return t > 0.f ? min(max(all_ones, 62 - (ilogbf(1.01f * t) + 1)), 61) : all_ones;
             };
             tc.bc = room(sx.h), tc.bo = room(sy.h);
         }
         __syncthreads();
         bc = tc.bc, bo = tc.bo;
     }
-    auto weight = [&](float u, float top, int e) -> D2 {
-        if (POWER) {
-            if (wide) {
-                const double v = u * inv_sigma;
-                return to_d2(ldexp(v * v + 1e-3, -e));
-            }
-            D2 v = is * D2{u, 0.f};
-            v = v * v + D2{1e-3f, (float)(1e-3 - (double)1e-3f)};
-            const float c = __int_as_float((127 - e) << 23);
-            return D2{v.h * c, v.l * c};
+    if (POWER) {
+        if (threadIdx.x == 0) {
+            // (u / sigma)^2 in the weights' units: u^2 times a factor of 53 bits
+            auto factor = [&](int bits, u64 &k, int &s, u64 &least) {
+                const u64 q = (u64)__double_as_longlong(ldexp(inv_sigma * inv_sigma, bits));
+                k = ((q & 0xfffffffffffffULL) | 0x10000000000000ULL) << 11;
+                s = 263 + 1075 - (int)(q >> 52);
+                least = __double2ull_rn(ldexp(1e-3, bits));
+            };
+            factor(bc - ec, tc.kc, tc.sc2, tc.least_c);
+            factor(bo - eo, tc.ko, tc.so2, tc.least_o);
         }
-        if (wide) return D2{expf((float)(((double)u - (double)top) * inv_sigma)), 0.f};
+        __syncthreads();
+    }
+    // A weight: kinds 1 and 3 in FP32; POWER in units (its 62 bits, from the
+    // exact square of u's 24)
+    auto weight = [&](float u, float top) -> float {
+        if (wide) return expf((float)(((double)u - (double)top) * inv_sigma));
         const D2 d = sum2(u, -top) * is;
-        return D2{expf(d.h + d.l), 0.f};
+        return expf(d.h + d.l);
     };
-    auto units = [&](D2 w, int bits) -> u64 {
-        u64 x = fixed_point(w.h, bits);
-        if (POWER) x = w.l < 0.f ? x - fixed_point(-w.l, bits) : x + fixed_point(w.l, bits);
-        return x;
+    auto power_units = [&](float u, u64 factor, int s, u64 least) -> u64 {
+        const unsigned b = __float_as_uint(u), e = b >> 23 & 0xffu;
+        const u64 m = (b & 0x7fffffu) | (e ? 0x800000u : 0u);
+        const int r = min(max(s - 2 * (int)max(e, 1u) - 1, 0), 63);  // (the last place rounds)
+        return (((__umul64hi(m * m << 16, factor) >> r) + 1) >> 1) + least;
     };
     const int k0 = min(n, (int)threadIdx.x * run), k1 = min(n, k0 + run);
 
@@ -519,11 +533,20 @@ __global__ void __maxnreg__(56) k_ot(OtArgs a, int run) {
     u64 F = 0, offG = 0;
     bool bad = POWER && inv_sigma == 0.0;  // (an infinite sigma, and with it every weight)
     for (int k = k0; k < k1; k++) {
-        const D2 x = weight(U[k], mc, ec), y = weight(O[k], mo, eo);
-        bad |= !(x.h <= 2.f && y.h <= 2.f);
-        if (!POWER) U[k] = x.h;
-        F += units(x, bc);
-        offG += units(y, bo);
+        const float u = U[k], v = O[k];
+        if (POWER) {
+            if (fabsf(u) == mc) atomicMin(&tc.kref, k);
+            bad |= !(fabsf(u) <= FLT_MAX && fabsf(v) <= FLT_MAX);
+            F += power_units(u, tc.kc, tc.sc2, tc.least_c);
+            offG += power_units(v, tc.ko, tc.so2, tc.least_o);
+        } else {
+            const float x = weight(u, mc), y = weight(v, mo);
+            bad |= !(x <= 2.f && y <= 2.f);
+            if (x == 1.f) atomicMin(&tc.kref, k);
+            U[k] = x;
+            F += fixed_point(x, bc);
+            offG += fixed_point(y, bo);
+        }
         G[k] = offG;
     }
     bad = __syncthreads_or(bad);
@@ -531,15 +554,28 @@ __global__ void __maxnreg__(56) k_ot(OtArgs a, int run) {
     for (int k = k0; k < k1; k++) G[k] += offG;
     if (threadIdx.x == 0) {
         const double sf = (double)ws[1][64], sg = (double)ws[1][65], q = sg / sf;
-        // ratio of the units, SG / SF = (ratio / 2^63) 2^shift
+        // ratio of the units, SG / SF = (ratio / 2^63) 2^shift, rounded up: F SG / SF
+        // rounds down to the integer wherever it is one (equal shapes have r = 0)
         const u64 rb = (u64)__double_as_longlong(q);
         tc.ratio = ((rb & 0xfffffffffffffULL) | 0x10000000000000ULL) << 11;
         tc.shift = (int)(rb >> 52) - 1023;
-        // f / g = (p / SF) (SG / g), p and g in their units
-        tc.c = to_d2(-2.0 * ldexp(q, bc));
-        // sums of weights are SF 2^-bc
+        if (abs(tc.shift) < 62) {
+            // (FP64's 53 bits, and the rest from the remainder)
+            const u64 s = ws[1][64];
+            __int128 d = ((unsigned __int128)ws[1][65] << (63 - tc.shift)) - (unsigned __int128)tc.ratio * s;
+            const int c = __float2int_rn(__ll2float_rn((long long)(d >> 32)) * __fdividef(4294967296.f, (float)s));
+            u64 r = tc.ratio + c;
+            d -= (__int128)c * s;
+            for (int i = 0; i < 4 && d > 0; i++, d -= s) r++;
+            for (int i = 0; i < 4 && d <= -(__int128)s; i++, d += s) r--;
+            tc.ratio = r;
+        }
+        // f / g = (p / SF) (SG / g), p and g in their units; sums of weights are
+        // SF 2^-bc (p of kinds 1, 3: without the 2^-bc)
         const double inv_S = ldexp(1.0 / sf, bc);
-        tc.norm = to_d2(-inv_S);
+        tc.c = to_d2(-2.0 * (POWER ? q : ldexp(q, bc)));
+        tc.inv_S = POWER ? 1.0 / sf : inv_S;
+        tc.norm = to_d2(-tc.inv_S);
         // res = (1/2) (A - FA) / S p'(u): p' = p / sigma, or (POWER, p in units
         // of 2^ec sigma^2) 2 (u / sigma) / sigma
         tc.scale = a.dt * a.dt * inv_S * (POWER ? ldexp(1.0, -ec) : 0.5);
@@ -552,24 +588,31 @@ __global__ void __maxnreg__(56) k_ot(OtArgs a, int run) {
         if (threadIdx.x == 0) a.trace_misfit[2 * tr + comp] = __longlong_as_double(0x7fffffffffffffffLL);
         return;
     }
-    auto p_of = [&](int k) -> D2 { return POWER ? weight(U[k], mc, ec) : D2{U[k], 0.f}; };
-
     // transport, in samples: r_k = k + 1 - T_k = i - (F_k - G_{m-1}) / g_m, i = k + 1 - m
     // Adjoint weights in samples squared: A_k = r_k^2 + c sum_{j>=k} q_j, q_j = r_j p_j / g_m(j).
     // The sum is the block's after this thread's samples, plus the thread's own less what
     // comes before k, so a thread keeps B_k = r_k^2 - c sum_{j<k} q_j and adds a
     // constant when the block's sums are known.
-    const u64 ratio = tc.ratio, SF = ws[1][64], SG = ws[1][65];
-    const int shift = tc.shift;
+    // Where one sample holds nearly all the weight, its A - FA is a small
+    // difference: FA is formed relative to A of the sample of the largest
+    // weight, kref, whose term is then none.
+    const int kref = tc.kref;
+    const u64 ratio = tc.ratio;
+    const int up = 1 + min(max(tc.shift, 0), 62), down = min(max(-tc.shift, 0), 63);
     const D2 c = tc.c;
     D2 w{0.f, 0.f}, sq{0.f, 0.f}, fb{0.f, 0.f}, sp{0.f, 0.f};
     int m = 0;
     for (int k = k0; k < k1; k++) {
-        const D2 pk = p_of(k);
-        F += units(pk, bc);
-        u64 y = __umul64hi(F << 1, ratio);
-        y = shift >= 0 ? y << min(shift, 63) : y >> min(-shift, 63);
-        if (F == SF) y = SG;  // (the ratio is rounded)
+        D2 pk;
+        if (POWER) {
+            const u64 x = power_units(U[k], tc.kc, tc.sc2, tc.least_c);
+            pk = to_d2(x);
+            F += x;
+        } else {
+            pk = D2{U[k], 0.f};
+            F += fixed_point(U[k], bc);
+        }
+        const u64 y = __umul64hi(F << up, ratio) >> down;
         m = first_above(G, n, y, m);
         const u64 below = m > 0 ? G[m - 1] : 0, g = G[m] - below;
         // (r of -1 to 1 from integers alone: near equal traces lose nothing)
@@ -580,21 +623,26 @@ __global__ void __maxnreg__(56) k_ot(OtArgs a, int run) {
         const D2 b = rr + -(c * sq);
         B[k] = b;
         w = w + pk * rr;
-        fb = fb + pk * b;
-        sp = sp + pk;
+        if (k != kref) {
+            fb = fb + pk * b;
+            sp = sp + pk;
+        }
         sq = sq + pk * r * ig;
     }
     const D2 rest = c * (block_suffix(sq, ws[0]) + sq);
-    fb = fb + rest * sp;
+    if (kref >= k0 && kref < k1) tc.ref = B[kref] + rest;
+    __syncthreads();
+    const D2 shift_a = rest + -tc.ref;  // A - A of kref = B + shift_a
+    fb = fb + shift_a * sp;
     block_sum2(fb, w, ws[1]);
     if (threadIdx.x == 0) {
         tc.FA = fb * tc.norm;
-        a.trace_misfit[2 * tr + comp] = -to_f64(w * tc.norm) * a.dt * a.dt;
+        a.trace_misfit[2 * tr + comp] = to_f64(w) * tc.inv_S * a.dt * a.dt;
     }
     __syncthreads();
     const D2 FA = tc.FA, sc = tc.sc;
     for (int k = k0; k < k1; k++) {
-        const D2 d = (B[k] + rest) + FA, x{U[k], 0.f};
+        const D2 d = k == kref ? FA : (B[k] + shift_a) + FA, x{U[k], 0.f};
         if (wide) {
             res[k] = (float)(to_f64(d) * tc.scale * (POWER ? inv_sigma * U[k] : U[k]) * inv_sigma);
         } else {
