@@ -121,13 +121,16 @@ __device__ __forceinline__ Cells cells_at(const AdjArgs &a) {
     return c;
 }
 
-// peak[0]: max |record|, peak[1]: max |background velocity| over every 16th step, as bits
+// peak[0]: max |record|, peak[1]: max |background velocity| over every 16th step
+// back from the last one that the stress part reads, as bits (a wave's amplitude
+// changes little in 16 steps once it is under way; of a run of a few steps
+// the last has it, the first may have none)
 __global__ void k_adj_peaks(const __grid_constant__ AdjArgs a, long long nrec) {
     float m = 0.f, v = 0.f;
     const long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
     for (long long i = i0; i < nrec; i += step) m = fmaxf(m, fmaxf(fabsf(a.dz[i]), fabsf(a.dx[i])));
     const long long n = (long long)2 * a.X * a.PS / 4;  // a step's velocities, four at a time
-    for (int it = 0; it < a.nt; it += 16) {
+    for (int it = a.nt - 2; it >= 0; it -= 16) {
         const float4 *q = reinterpret_cast<const float4 *>(a.snap + (size_t)it * 2 * a.X * a.PS);
         for (long long i = i0; i < n; i += step) {
             const float4 w = q[i];
