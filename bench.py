@@ -407,6 +407,19 @@ def observed_records(sg, w, data):
     return obs
 
 
+def step_kernels(sweeps, ways, born, snap_fmt, fwd_ms, bwd_ms):
+    """ms a launch of the kernels that the timed passes ran: `sweeps`, the four
+    sweeps timed by themselves, less those of a direction that took whole steps
+    (`ways`, FD2DGPU_ELASTIC.debug_steps), whose step's time is its share of that
+    phase of the passes."""
+    kt = {k: v for k, v in sweeps.items() if ways["k_bwd" in k] == "sweeps"}
+    if ways[0] != "sweeps":
+        kt["k_%s_fwd%s" % (ways[0], "<born>" if born else "")] = fwd_ms
+    if ways[1] != "sweeps":
+        kt["k_%s_bwd%s" % (ways[1], "<%s>" % snap_fmt if snap_fmt else "")] = bwd_ms
+    return kt
+
+
 def measure(w, args, steps, warmup, plain_shots, pg=None, ws=1, rank=0, clocks=None, snap_check=0):
     """One workload: `warmup` untimed passes (the autotuner after the first),
     then `steps` timed passes through sfwi_run (device time from CUDA events
@@ -532,17 +545,14 @@ def measure(w, args, steps, warmup, plain_shots, pg=None, ws=1, rank=0, clocks=N
     d2h = 3 * w["allnx"] * w["allnz"] * 4 + 8 * len(shots) + (8 * w["allnx"] * w["allnz"] if w.get("rho_grad") else 0)
 
     # per-kernel average launch durations (CUDA events on the engine stream)
-    kt = fd.time_kernels(reps=20)
-    if launches < 2.9 * nt * steps:
-        # both directions ran whole steps per launch, not the four sweeps
-        # that were just timed: a step's time from its phase of the passes
-        snap = "<%s>" % w["snap"][1] if w.get("snap") else ""
-        kt = {"k_march_fwd<born>" if fd.stage == 2 else "k_march_fwd": float(np.mean(fwd_ms)) / nt,
-              "k_march_bwd" + snap: float(np.mean(bwd_ms)) / nt}
+    ways = fd.debug_steps()
+    kt = step_kernels(fd.time_kernels(reps=20), ways, fd.stage == 2, w["snap"][1] if w.get("snap") else None,
+                      float(np.mean(fwd_ms)) / nt, float(np.mean(bwd_ms)) / nt)
     peak, peak_kind = measured_peak_hbm()
     cells = sum((d["nx"] + 2 * pml) * nzpml for d in shots)
     roof, fracs = None, None
     if kt:
+        kbytes.update({k.replace("march", "burst"): v for k, v in kbytes.items()})
         fracs = {k: round(kbytes[k] * cells / (v / 1000.0) / 1e9 / peak, 4) for k, v in kt.items()}
         dom = max(kt, key=kt.get)
         achieved = kbytes[dom] * cells / (kt[dom] / 1000.0) / 1e9
