@@ -856,6 +856,10 @@ void march_items(const sfwi_handle *h, const MarchVariant &w, int slots, std::ve
                 m.g = g;
                 const int v0 = m.x0 - 8, v1 = v0 + ((m.x1 - m.x0 + 3) / 4 + 4) * 4;
                 if (g.isx >= v0 && g.isx < v1 && g.isz >= m.z0 - 8 && g.isz < m.z0 - 8 + ps) m.flags |= MARCH_SOURCE;
+                // (below the update region only where a vertical force enters the
+                // stress half-step's view there)
+                const bool below = h->src_kind == SRC_VZ_FORCE && (m.flags & MARCH_SOURCE) && g.isz >= g.nzpml - NOP;
+                m.vend = below ? g.nzpml : std::min(m.z0 + m.zw + NOP, g.nzpml - NOP);
                 if (g.ntr > 0 && g.igz >= m.z0 - 8 && g.igz < m.z0 - 8 + ps) m.flags |= MARCH_RECV;
                 items.push_back(m);
                 per_shot[s]++;

@@ -45,8 +45,9 @@ enum MarchFlags : int {
 };
 struct alignas(16) MarchItem {
     int shot, x0, x1, z0, zw, flags;
+    int vend;  // the forward velocity half-step's columns of use end here
     ShotGeo g;
-    int pad[3];
+    int pad[2];
 };
 static_assert(sizeof(MarchItem) == 80, "MarchItem is five 16-byte words");
 // Fields advance from one copy to the other; two fields that advance together
