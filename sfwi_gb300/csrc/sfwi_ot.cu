@@ -633,6 +633,7 @@ __global__ void __maxnreg__(56) k_ot(OtArgs a, int run) {
     if (kref >= k0 && kref < k1) tc.ref = B[kref] + rest;
     __syncthreads();
     const D2 shift_a = rest + -tc.ref;  // A - A of kref = B + shift_a
+    if (kref >= k0 && kref < k1) B[kref] = -shift_a;  // (its difference: none, exactly)
     fb = fb + shift_a * sp;
     block_sum2(fb, w, ws[1]);
     if (threadIdx.x == 0) {
@@ -642,7 +643,7 @@ __global__ void __maxnreg__(56) k_ot(OtArgs a, int run) {
     __syncthreads();
     const D2 FA = tc.FA, sc = tc.sc;
     for (int k = k0; k < k1; k++) {
-        const D2 d = k == kref ? FA : (B[k] + shift_a) + FA, x{U[k], 0.f};
+        const D2 d = (B[k] + shift_a) + FA, x{U[k], 0.f};
         if (wide) {
             res[k] = (float)(to_f64(d) * tc.scale * (POWER ? inv_sigma * U[k] : U[k]) * inv_sigma);
         } else {
