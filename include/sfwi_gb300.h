@@ -365,8 +365,8 @@ int sfwi_set_source(sfwi_handle *h, int kind);
 
 /* Bytes that the copies of the wavefields of whole time steps (below) may take
  * in later runs of this handle, beside the device's own limit, an eighth of what
- * is free.  Runs that would need more take the sweeps, with the same results;
- * 0: never a copy.  A program that shares the device by a budget counts what
+ * is free.  Runs that would need more take the sweeps, backward at least, with
+ * the same results; 0: never a copy.  A program that shares the device by a budget counts what
  * it allows here.  Default: no limit. */
 int sfwi_set_copy_limit(sfwi_handle *h, size_t bytes);
 /* Select the tile shape for this handle's runs, which then take the four

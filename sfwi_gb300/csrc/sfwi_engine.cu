@@ -963,20 +963,29 @@ int upload_march(sfwi_handle *h, bool forward_only) {
     Batch &b = h->b;
     if (b.grid2.n * sizeof(float) > h->copy_limit) b.grid2.release();
     if (!b.way[0] && !b.way[1]) return SFWI_OK;
-    const size_t n = layout_march(h, forward_only), nf = b.items[0].size(), nb = b.items[1].size();
     // (the items first: they may have an earlier run's copy given back)
-    bool have = b.ditems.ensure(nf + nb) == cudaSuccess;
+    bool have = b.ditems.ensure(b.items[0].size() + b.items[1].size()) == cudaSuccess;
+    size_t n = layout_march(h, forward_only);
     if (have && !(n <= b.grid2.n && b.grid2.p)) {
-        size_t free_bytes = 0, total = 0;
+        size_t room = 0, total = 0;
         b.grid2.release();
-        CK(cudaMemGetInfo(&free_bytes, &total));
-        free_bytes = std::min(free_bytes, h->mem.limit - std::min(h->mem.used, h->mem.limit));
-        have = n * sizeof(float) <= std::min(free_bytes / 8, h->copy_limit) && b.grid2.ensure(n) == cudaSuccess;
+        CK(cudaMemGetInfo(&room, &total));
+        room = std::min(room, h->mem.limit - std::min(h->mem.used, h->mem.limit)) / 8;
+        room = std::min(room, h->copy_limit) / sizeof(float);
+        if (n > room && b.way[0] && b.way[1]) {
+            // plain forward steps by themselves need an eleventh of it
+            b.way[1] = nullptr;
+            b.items[1].clear();
+            b.items_active[1].clear();
+            n = layout_march(h, forward_only);
+        }
+        have = n <= room && b.grid2.ensure(n) == cudaSuccess;
     }
     if (!have) {
         no_march(b);
         return SFWI_OK;
     }
+    const size_t nf = b.items[0].size(), nb = b.items[1].size();
     layout_march(h, forward_only);  // now with the buffer in place
     CK(cudaMemsetAsync(b.grid2.p, 0, n * sizeof(float), h->st));
     if (nf) CK(cudaMemcpyAsync(b.ditems.p, b.items[0].data(), nf * sizeof(MarchItem), cudaMemcpyHostToDevice, h->st));

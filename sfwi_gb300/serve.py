@@ -114,13 +114,13 @@ def batch_bytes(reqs, strip_chunk=0):
     return 4 * floats + 8 * 4 * cells + (1 << 20)
 
 
-def copy_bytes(reqs):
-    """The most that the copies of the wavefields of whole time steps take in
-    one run of the requests: 44 arrays of the packed grid (layout_march,
-    sfwi_engine.cu, stage 1)."""
+def copy_bytes(reqs, arrays=44):
+    """What the copies of the wavefields of whole time steps take in one run of
+    the requests at most: 44 arrays of the packed grid, 4 where only the
+    forward steps have them (layout_march, sfwi_engine.cu, stage 1)."""
     pml = reqs[0].pml
     P = (max(r.allnz for r in reqs) + 2 * pml + 3) // 4 * 4
-    return 4 * 44 * P * sum(int(d["nx"]) + 2 * pml for r in reqs for d in r.shots)
+    return 4 * arrays * P * sum(int(d["nx"]) + 2 * pml for r in reqs for d in r.shots)
 
 
 def run_requests(reqs, strip_chunk=0, copy_limit=None):
@@ -268,8 +268,8 @@ class Server:
 
         def copies(group, left):
             # what the group's run may take beside its own size, of `left` bytes
-            need = copy_bytes(group) if self.own_runner else 0
-            return need if 8 * need <= left else 0
+            fit = [c for c in (copy_bytes(group), copy_bytes(group, 4)) if 8 * c <= left] if self.own_runner else []
+            return fit[0] if fit else 0
 
         def worker(group, size, admitted, copy):
             arg = (copy,) if self.own_runner else ()
