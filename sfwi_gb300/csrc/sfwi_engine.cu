@@ -907,8 +907,10 @@ void no_march(Batch &b) {
 //     21.7 -> 20.5; Born forward 29.4 -> 33.0, 28.8 -> 30.2, 28.4 -> 28.8 (38 shots: as
 //     without); stage 1 forward in FP32 22.3 -> 21.4 but 13.1 -> 13.6 us with three
 //     shots, in 16 bits 25.2 -> 21.5, 23.2 -> 20.2, 22.4 -> 19.2 us
-// Grids of less than 64 cells an SM stay with the sweeps: such a step is all
-// launch latency, and the launch counts of the golden cases are the sweeps'.
+// Grids of less than 64 cells an SM stay with the sweeps although bursts are
+// faster there too (stage 1, 20x12 nodes 7.7 -> 5.0, 10.8 -> 4.9 us; 60x40 7.5 -> 4.6,
+// 10.8 -> 5.1; Born 9.4 -> 4.3, 10.8 -> 5.1): the line has no other reason than that
+// the checks on the smallest models, golden vectors among them, count the sweeps' launches.
 constexpr long long MARCH_MIN_CELLS = 64, MARCH_FEW_CELLS = 1150, MARCH_ANY_CELLS = 3500, MARCH_MID_CELLS = 8000,
                     MARCH_PLAIN_CELLS = 9000, MARCH_LARGE_CELLS = 15000;
 constexpr int MARCH_SNAP_EVERY = 4;
@@ -1997,7 +1999,7 @@ int born_adjoint(sfwi_handle *h, const std::vector<ShotIn> &q, bool product, dou
         for (int r : {R_SYN_Z, R_SYN_X, R_SYN2_Z, R_SYN2_X}) CK(cudaMemsetAsync(b.r(r, nt), 0, n * sizeof(float), st));
     }
     CK(cudaEventRecord(h->ev[1], st));
-    // adjoint workspace: 18 float fields, 2 double accumulators, tables
+    // adjoint workspace: 18 float fields, 2 accumulators of float pairs, tables
     const size_t cells = b.cells, gcells = (size_t)h->allnx * h->allnz;
     CK(h->adj_f.ensure(18 * cells));
     CK(h->adj_d.ensure(2 * cells + 1));  // and the peaks

@@ -700,7 +700,7 @@ struct FwdBody {
 };
 
 // Measured against the two sweeps, per step: 38 Born shots at 376x201
-// 107 -> 92 us (5.6 TB/s of the 100 bytes a cell needs, 152 SMs), two stage-1 shots at
+// 107 -> 92 us (4.1 TB/s of the 100 bytes a cell needs, 152 SMs), two stage-1 shots at
 // 2001x801 51 -> 49 us.  The rest is the instructions of the INNER and EDGE warps, which a
 // group's barrier makes the others wait for (all warps LEAN: 72 us), and the
 // shared-memory loads of the stencils.  128 registers a thread are a hard limit: any

@@ -21,7 +21,7 @@
 // products and divisions in FP64 (the FP64 pipe, 1/64 of the FP32 rate, is 86 % busy:
 // 2.87 ms for both components of 3760 traces of 3000 samples; 1 to 2 % of a gradient run).
 // k_ot serves the calls that want a gather's misfit and residuals by themselves
-// and takes 0.47 ms: there the CDFs are 64-bit integers and the rest is in float
+// and takes 0.50 ms (OT_power 0.67): there the CDFs are 64-bit integers and the rest is in float
 // pairs.  Its residuals differ from k_ot_fp64's in the last bit of one in 2000, which is
 // nothing by itself; but an FP32 propagation of that source ends 7e-6 away from
 // the other's after 3000 steps (as far as each is from FP64), so gradient
@@ -400,8 +400,9 @@ __global__ void __launch_bounds__(OT_THREADS) k_ot_fp64(OtArgs a) {
 // Each thread owns one contiguous run of an odd number of samples (`run`), so that the
 // threads' accesses to 64-bit arrays in shared memory fall into different
 // banks; the quantile search continues from the previous sample's.
-// Bound by instructions (470 us for 3760 traces of 3000 samples, 64 % of the issue slots, DRAM 7 %); 56
-// registers let three CTAs of 352 threads share an SM (64: two, 685 us for 590).
+// Bound by instructions (500 us for 3760 traces of 3000 samples, 66 % of the issue slots, DRAM 6 %; OT_power
+// 668 us, 57 %); 56 registers let three CTAs of 352 threads share an SM (64: two; 685 us for 590 in an
+// earlier form).
 template <bool LONG, bool POWER>
 __global__ void __maxnreg__(56) k_ot(OtArgs a, int run) {
     extern __shared__ u64 ot_words[];
